@@ -542,12 +542,10 @@ int dfm_ilu_set_sweep_warps(dfm_ilu M, int compute_warps, int lanes, int produce
   if (!M || (compute_warps != 1 && compute_warps != 2 && compute_warps != 4) ||
       (lanes != 2 && lanes != 4 && lanes != 8) || producer_warps < 1 || compute_warps + producer_warps > 16)
     return DFM_ERR_INVALID;
-  if (M->sweep != 3 || !M->plan_f.halo) return DFM_ERR_INVALID;  // mode 9 only
-  for (SweepPlan* P : {&M->plan_f, &M->plan_b, &M->plan32_f, &M->plan32_b}) {
-    P->cw = compute_warps;
-    P->lpr = lanes;
-    P->hw = producer_warps;
-  }
+  if (M->sweep != 3 || !M->plan_f.halo) return DFM_ERR_INVALID;  // modes 9 and 10 only
+  const int rc = ilu_set_halo_shape(M, lanes, compute_warps);
+  if (rc) return rc;
+  for (SweepPlan* P : {&M->plan_f, &M->plan_b, &M->plan32_f, &M->plan32_b}) P->hw = producer_warps;
   M->plan_gen++;  // captured solves hold the old launch shape
   return DFM_OK;
 }
@@ -588,6 +586,7 @@ int dfm_ilu_set_sweep_partition(dfm_ilu M, const unsigned* part, unsigned nparts
     M->part_of.clear();
     M->nparts = 0;
   }
+  M->own_for = 0;
   M->sweep = 0;  // autotuned again on next use
   M->plan_gen++;
   return DFM_OK;

@@ -115,6 +115,8 @@ struct dfm_ilu_s {
   int fill_level = 0;
   std::vector<unsigned> part_of;  // optional row partition for the range sweeps: part of every row
   unsigned nparts = 0;
+  std::vector<unsigned> own_of;   // the partition by chains (sweep_part.cu) made for own_for parts
+  unsigned own_n = 0, own_for = 0;
   unsigned N = 0, b = 1, ncrs = 0;
   int vt = DFM_REAL;
   unsigned* d_diaind = nullptr;
@@ -193,14 +195,22 @@ int set_poll_sleep(unsigned ns);
 // sweep.cu
 // merge: steps are pairs of levels (the second level's operands on the
 // first are substituted by products with the factor; see sweep.cu)
-// part: the CTAs are the parts of the ILU's row partition (G must be its
-// part count) instead of balanced ranges of the natural row order
-// halo: the plan of the shared-memory-only schedule (sweep_halo.cu; unmerged,
-// FP64 vectors)
+// part: 1 the CTAs are the parts of the ILU's row partition (G must be its
+// part count), 2 (halo plans) those of its partition by chains for G parts,
+// 0 balanced ranges of the natural row order
+// halo: the plan of the shared-memory-only schedule (sweep_halo.cu; FP64
+// vectors), whose layout depends on the lanes per component lpr and the compute
+// warps cw (0: a default)
 int sweep_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, int vec_bytes, SweepPlan* P, bool merge = false,
-                     bool part = false, bool halo = false);
+                     int part = 0, bool halo = false, int lpr = 0, int cw = 0);
 // sweep_halo.cu
-int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* P, bool part, bool merge = false);
+// sweep_part.cu
+int sweep_own_partition(dfm_ilu M, unsigned G);
+int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* P, int part, bool merge, int H,
+                          int cw);
+int sweep_halo_refresh(dfm_ilu M, SweepPlan* P);
+// the halo plans of M rebuilt for other lanes per component and compute warps
+int ilu_set_halo_shape(dfm_ilu M, int lpr, int cw);
 cudaError_t sweep_halo_launch(dfm_ilu M, bool fwd, const SweepPlan* P, const double* in, double* out,
                               const double* rdot, double* part, KrylovScalars* sc, const double* rr_part, int rr_n,
                               bool f32);

@@ -828,7 +828,9 @@ int ilu_prepare(dfm_ilu M, bool f32) {
       SweepPlan& P32 = f ? M->plan32_b : M->plan32_f;
       if (!P32.valid || P32.G != P64.G || P32.lpr != P64.lpr || P32.merged != P64.merged ||
           P32.halo != P64.halo || P32.cw != P64.cw || P32.hw != P64.hw) {
-        if ((rc = sweep_plan_build(M, f == 0, P64.G, 4, 8, &P32, P64.merged, P64.part, P64.halo))) return rc;
+        const int G = P64.part == 2 ? P64.parts : P64.G;
+        if ((rc = sweep_plan_build(M, f == 0, G, 4, 8, &P32, P64.merged, P64.part, P64.halo, P64.lpr, P64.cw)))
+          return rc;
         P32.lpr = P64.lpr;
         P32.cw = P64.cw;
         P32.hw = P64.hw;
@@ -882,177 +884,115 @@ int ilu_autotune(dfm_ilu M) {
     if (rc) return rc;
     if (ms < best) { best = ms; best_mode = mode; }
   }
-  // range-partitioned schedule: every CTA count whose slice fits in shared memory,
-  // then, at the best count, merged level pairs and the barrier-free kernel
-  // (complex matrices run as real 2x2 blocks)
+  // The shared-memory-only schedule (modes 9 and 10; complex matrices run as
+  // real 2x2 blocks).  Building a plan's level data costs more than timing it,
+  // so the candidates go coordinate by coordinate: row partitions and CTA
+  // counts first, at the lanes and compute warps that a level's rows suggest,
+  // then other warps and lanes at the best of them, then merged level pairs.
+  // (The range schedules 3-8 were slower than this one on every system timed:
+  // 2-D Poisson 256^2, an application 412 us by mode 8 against 184 us by mode
+  // 9; they remain for callers that ask for them.)
   {
     sweep_plan_free(&M->plan_f);
     sweep_plan_free(&M->plan_b);
     SweepPlan best_f, best_b;  // owned here until the end
     const int nsm = M->ctx->nsm;
-    const int cand[] = {nsm, nsm / 2, nsm / 4, 16, 8, 4, 2, 1};
-    int last = -1, best_G = 0;
-    float best3 = 1e30f;
-    // times the candidate plans (pf, pb) over lanes per row and the kernel
-    // variants in `kinds` (0 = level barrier, 1 = barrier-free, 2 = level
-    // barrier with the two-half row pipeline); keeps them in best_f/best_b if
-    // they beat `best`
-    auto try_plans = [&](SweepPlan& pf, SweepPlan& pb, std::initializer_list<int> kinds, float* tbest) -> int {
-      std::swap(M->plan_f, pf);  // M holds the candidate
-      std::swap(M->plan_b, pb);
-      float ms = 1e30f;
-      int rc = DFM_OK, best_lpr = 1, best_kind = 0;
-      for (int kind : kinds) {
-        if (rc) break;
-        if (kind == 1 && !(M->plan_f.nb_ok && M->plan_b.nb_ok)) continue;
-        for (int lpr : {1, 2, 4, 8}) {  // consumer lanes per row
-          M->plan_f.lpr = M->plan_b.lpr = lpr;
-          M->plan_f.nb = M->plan_b.nb = kind == 1;
-          M->plan_f.pipe = M->plan_b.pipe = kind == 2;
-          float t = 1e30f;
-          rc = time_mode(3, &t);
-          if (rc) break;
-          if (t < ms) { ms = t; best_lpr = lpr; best_kind = kind; }
-        }
-      }
-      M->plan_f.lpr = M->plan_b.lpr = best_lpr;
-      M->plan_f.nb = M->plan_b.nb = best_kind == 1;
-      M->plan_f.pipe = M->plan_b.pipe = best_kind == 2;
-      std::swap(M->plan_f, pf);  // candidate back in pf/pb, M empty
-      std::swap(M->plan_b, pb);
-      if (tbest) *tbest = ms;
-      if (rc == DFM_OK && ms < best) {
-        best = ms;
-        best_mode = 3;
-        sweep_plan_free(&best_f);
-        sweep_plan_free(&best_b);
-        std::swap(best_f, pf);
-        std::swap(best_b, pb);
-      } else {
-        sweep_plan_free(&pf);
-        sweep_plan_free(&pb);
-      }
-      return rc;
+    const unsigned bx = M->vt == DFM_COMPLEX ? 2u : M->b;
+    const unsigned nlev = std::max(1u, std::max(M->nlev_f, M->nlev_b));
+    struct Cand {
+      int part, G, lpr, cw;
+      bool merge;
     };
-    // the caller's row partition (one CTA per part) first, then balanced
-    // ranges of the natural order at every CTA count
-    bool best_part = false;
-    auto try_G = [&](int G, bool part) -> int {
+    Cand top = {0, 0, 0, 0, false};
+    float top_ms = 1e30f;
+    int err = DFM_OK;
+    // builds and times a candidate; false if it cannot be built
+    auto eval = [&](const Cand& c) {
       SweepPlan pf, pb;
-      if (sweep_plan_build(M, true, G, 8, 8, &pf, false, part) != DFM_OK ||
-          sweep_plan_build(M, false, G, 8, 8, &pb, false, part) != DFM_OK) {
+      if (sweep_plan_build(M, true, c.G, 8, 8, &pf, c.merge, c.part, true, c.lpr, c.cw) != DFM_OK ||
+          sweep_plan_build(M, false, c.G, 8, 8, &pb, c.merge, c.part, true, c.lpr, c.cw) != DFM_OK) {
         sweep_plan_free(&pf);
         sweep_plan_free(&pb);
         cudaGetLastError();
-        return DFM_OK;  // slice does not fit in shared memory at this CTA count
+        return;
       }
-      float t = 1e30f;
-      const int rc = try_plans(pf, pb, {0, 2}, &t);
-      if (rc != DFM_OK && rc != DFM_ERR_UNSUPPORTED) return rc;
-      if (rc == DFM_OK && t < best3) { best3 = t; best_G = G; best_part = part; }
-      return DFM_OK;
+      pf.hw = pb.hw = 9 - c.cw;  // every warp the launch has left polls halo rows
+      std::swap(M->plan_f, pf);  // M holds the candidate
+      std::swap(M->plan_b, pb);
+      float ms = 1e30f;
+      const int rc = time_mode(3, &ms);
+      std::swap(M->plan_f, pf);
+      std::swap(M->plan_b, pb);
+      if (rc != DFM_OK && rc != DFM_ERR_UNSUPPORTED && err == DFM_OK) err = rc;
+      if (rc == DFM_OK && ms < top_ms) {
+        top_ms = ms;
+        top = c;
+        std::swap(best_f, pf);
+        std::swap(best_b, pb);
+      }
+      sweep_plan_free(&pf);
+      sweep_plan_free(&pb);
     };
-    if (M->nparts > 0 && M->nparts <= (unsigned)nsm) {
-      const int rc = try_G((int)M->nparts, true);
-      if (rc) {
-        sweep_plan_free(&best_f);
-        sweep_plan_free(&best_b);
-        return rc;
+    // rows whose blocks do not fit the lanes' registers take the slower kernel for longer rows
+    unsigned long_rows = 0;
+    for (unsigned i = 0; i < M->N; i++) {
+      const unsigned nb = M->h_diaind[i] - M->A->h_rowptr[i], nu = M->A->h_rowptr[i + 1] - M->h_diaind[i];
+      long_rows = std::max(long_rows, std::max(nb, nu));
+    }
+    const int h0 = bx == 3 ? (long_rows > 8 ? 4 : 2) : (long_rows > 3 ? 2 : 1);
+    const unsigned rpw = 32u / (bx * (unsigned)h0);
+    auto warps_for = [&](int G) {  // a level's rows of one CTA in one round
+      const double rows = 1.2 * M->N / ((double)G * nlev);
+      return rows <= rpw ? 1 : rows <= 2.0 * rpw ? 2 : 4;
+    };
+    const bool large = M->N > 150000;  // a plan takes tenths of a second there
+    if (M->nparts > 0 && M->nparts <= (unsigned)nsm) eval({1, (int)M->nparts, h0, warps_for((int)M->nparts), false});
+    const int counts[] = {nsm, 64, 32, 24, 16, 12, 8, 6, 4, 2, 1};
+    float last = 1e30f;
+    int worse = 0;
+    for (int G : counts) {
+      if (err || worse > 1 || (large && G < 64)) break;
+      if (G > nsm || (G > 1 && M->N < 64u * (unsigned)G)) continue;
+      const float before = top_ms;
+      eval({2, G, h0, warps_for(G), false});
+      if (!large || G == nsm) eval({0, G, h0, warps_for(G), false});
+      worse = before < 1e29f && top_ms == before && last < 1e29f ? worse + 1 : 0;
+      last = top_ms;
+    }
+    if (top.G) {
+      Cand c = top;
+      for (int cw : {1, 2, 4})
+        if (!err && cw != c.cw && (!large || cw > c.cw / 2)) {
+          Cand d = top;
+          d.cw = cw;
+          eval(d);
+        }
+      if (!err) {
+        Cand d = top;
+        d.lpr = bx == 3 ? 6 - top.lpr : 3 - std::min(top.lpr, 2);  // 2 <-> 4, 1 <-> 2
+        d.cw = d.lpr > top.lpr ? std::min(4, 2 * top.cw) : std::max(1, top.cw / 2);
+        eval(d);
+      }
+      if (!err && !large) {
+        Cand d = top;
+        d.merge = true;
+        if (bx < 3) d.lpr = 2;  // a merged row has about twice the blocks
+        eval(d);
       }
     }
-    for (int G : cand) {
-      if (G < 1 || G == last) continue;
-      last = G;
-      const int rc = try_G(G, false);
-      if (rc) {
-        sweep_plan_free(&best_f);
-        sweep_plan_free(&best_b);
-        return rc;
-      }
+    if (err) {
+      sweep_plan_free(&best_f);
+      sweep_plan_free(&best_b);
+      return err;
     }
-    if (best_G > 0) {
-      for (int mg = 0; mg < 2; mg++) {  // barrier-free kernel unmerged, then merged pairs with every kernel
-        SweepPlan pf, pb;
-        if (sweep_plan_build(M, true, best_G, 8, 8, &pf, mg != 0, best_part) != DFM_OK ||
-            sweep_plan_build(M, false, best_G, 8, 8, &pb, mg != 0, best_part) != DFM_OK) {
-          sweep_plan_free(&pf);
-          sweep_plan_free(&pb);
-          cudaGetLastError();
-          continue;
-        }
-        const int rc = mg ? try_plans(pf, pb, {0, 1, 2}, nullptr) : try_plans(pf, pb, {1}, nullptr);
-        if (rc != DFM_OK && rc != DFM_ERR_UNSUPPORTED) {
-          sweep_plan_free(&best_f);
-          sweep_plan_free(&best_b);
-          return rc;
-        }
-      }
+    if (top_ms < best) {
+      best = top_ms;
+      best_mode = 3;
+      std::swap(M->plan_f, best_f);
+      std::swap(M->plan_b, best_b);
     }
-    // the shared-memory-only schedule (modes 9 and 10) at the partition and at
-    // one CTA per SM: compute warps x lanes per row, producer warps
-    {
-      const unsigned bx = M->vt == DFM_COMPLEX ? 2u : M->b;
-      struct Cfg { int cw, lpr, hw; };
-      const Cfg cfgs3[] = {{1, 4, 4}, {2, 4, 4}, {4, 4, 4}, {4, 8, 4}, {2, 8, 4}, {4, 4, 8}};
-      const Cfg cfgs1[] = {{1, 2, 4}, {1, 4, 4}, {2, 4, 4}, {4, 4, 4}, {2, 2, 4}, {4, 4, 8}};
-      const Cfg* cfgs = bx == 1 ? cfgs1 : cfgs3;
-      auto try_halo = [&](int G, bool part, bool merge) -> int {
-        SweepPlan pf, pb;
-        if (sweep_plan_build(M, true, G, 8, 8, &pf, merge, part, true) != DFM_OK ||
-            sweep_plan_build(M, false, G, 8, 8, &pb, merge, part, true) != DFM_OK) {
-          sweep_plan_free(&pf);
-          sweep_plan_free(&pb);
-          cudaGetLastError();
-          return DFM_OK;
-        }
-        std::swap(M->plan_f, pf);
-        std::swap(M->plan_b, pb);
-        float ms = 1e30f;
-        Cfg bc = cfgs[0];
-        int rc = DFM_OK;
-        for (int q = 0; q < 6 && rc == DFM_OK; q++) {
-          M->plan_f.cw = M->plan_b.cw = cfgs[q].cw;
-          M->plan_f.lpr = M->plan_b.lpr = cfgs[q].lpr;
-          M->plan_f.hw = M->plan_b.hw = cfgs[q].hw;
-          float t = 1e30f;
-          rc = time_mode(3, &t);
-          if (rc == DFM_OK && t < ms) { ms = t; bc = cfgs[q]; }
-          if (rc == DFM_ERR_CUDA || rc == DFM_ERR_UNSUPPORTED) {  // a launch this configuration cannot have
-            cudaGetLastError();
-            rc = DFM_OK;
-          }
-        }
-        M->plan_f.cw = M->plan_b.cw = bc.cw;
-        M->plan_f.lpr = M->plan_b.lpr = bc.lpr;
-        M->plan_f.hw = M->plan_b.hw = bc.hw;
-        std::swap(M->plan_f, pf);
-        std::swap(M->plan_b, pb);
-        if (rc == DFM_OK && ms < best) {
-          best = ms;
-          best_mode = 3;
-          sweep_plan_free(&best_f);
-          sweep_plan_free(&best_b);
-          std::swap(best_f, pf);
-          std::swap(best_b, pb);
-        } else {
-          sweep_plan_free(&pf);
-          sweep_plan_free(&pb);
-        }
-        return rc == DFM_ERR_UNSUPPORTED ? DFM_OK : rc;
-      };
-      int rc = DFM_OK;
-      for (int mg = 0; mg < 2 && rc == DFM_OK; mg++) {  // levels one by one (mode 9), in merged pairs (mode 10)
-        if (M->nparts > 0 && M->nparts <= (unsigned)nsm) rc = try_halo((int)M->nparts, true, mg != 0);
-        if (rc == DFM_OK) rc = try_halo(nsm, false, mg != 0);
-      }
-      if (rc) {
-        sweep_plan_free(&best_f);
-        sweep_plan_free(&best_b);
-        return rc;
-      }
-    }
-    std::swap(M->plan_f, best_f);
-    std::swap(M->plan_b, best_b);
+    sweep_plan_free(&best_f);
+    sweep_plan_free(&best_b);
     M->plan_gen++;
   }
   cudaEventDestroy(e0);
@@ -1067,7 +1007,7 @@ int ilu_autotune(dfm_ilu M) {
 
 int ilu_set_ranges(dfm_ilu M, int G, bool merge, bool halo) {
   SweepPlan pf, pb;
-  const bool part = M->nparts > 0;  // a row partition, when set, fixes the CTAs
+  const int part = M->nparts > 0 ? 1 : 0;  // a row partition, when set, fixes the CTAs
   if (part) G = (int)M->nparts;
   int rc = sweep_plan_build(M, true, G, 8, 8, &pf, merge, part, halo);
   if (!rc) rc = sweep_plan_build(M, false, G, 8, 8, &pb, merge, part, halo);
@@ -1081,6 +1021,27 @@ int ilu_set_ranges(dfm_ilu M, int G, bool merge, bool halo) {
   std::swap(M->plan_f, pf);
   std::swap(M->plan_b, pb);
   M->sweep = 3;
+  M->plan_gen++;
+  return DFM_OK;
+}
+
+int ilu_set_halo_shape(dfm_ilu M, int lpr, int cw) {
+  if (M->plan_f.lpr == lpr && M->plan_b.lpr == lpr && M->plan_f.cw == cw && M->plan_b.cw == cw) return DFM_OK;
+  SweepPlan pf, pb;
+  const SweepPlan& P = M->plan_f;
+  const int G = P.part == 2 ? P.parts : P.G;
+  int rc = sweep_plan_build(M, true, G, 8, 8, &pf, P.merged, P.part, true, lpr, cw);
+  if (!rc) rc = sweep_plan_build(M, false, G, 8, 8, &pb, P.merged, P.part, true, lpr, cw);
+  if (rc) {
+    sweep_plan_free(&pf);
+    sweep_plan_free(&pb);
+    return rc;
+  }
+  DFM_CUDA_TRY(cudaStreamSynchronize(M->ctx->stream));
+  sweep_plan_free(&M->plan_f);
+  sweep_plan_free(&M->plan_b);
+  std::swap(M->plan_f, pf);
+  std::swap(M->plan_b, pb);
   M->plan_gen++;
   return DFM_OK;
 }

@@ -612,31 +612,9 @@ k_sweep_ranges_nb(const ChunkDesc* __restrict__ chunks, const unsigned* __restri
     }
 }
 
-// Refreshes the blob's values from the factor after a numeric factorisation.
-// Every packed block has a recipe {base, t0, t1, sign}:
-//   value = (base != NONE ? F[base] : 0) + sign * sum_{t0 <= t < t1} F[s1] (D_j^-1) (F[s2])
-// with a term {s1, j, s2} (j or s2 NONE = identity), F the factor's off-diagonal
-// blocks.  Plain operands are copies (no terms); the merged plans' operands of
-// the second level of a pair are the products L_ij D_j^-1 (forward input
-// terms), U'_ij (backward input terms) and the fill blocks
-// F_ik - sum_j F_ij (D_j^-1) F_jk.  One thread per packed block; D^-1 rows of the
-// forward sweep are copied alongside.  CPLX: the factor holds complex scalars
-// (re, im), packed as the real 2x2 blocks [re -im; im re] (B = 2), whose
-// products are the complex products.
-template <int B, bool CPLX>
-DFM_DEVINL void load_factor_blk(const double* __restrict__ src, size_t k, double* v) {
-  if constexpr (CPLX) {
-    const double re = src[2 * k], im = src[2 * k + 1];
-    v[0] = re;
-    v[1] = -im;
-    v[2] = im;
-    v[3] = re;
-  } else {
-#pragma unroll
-    for (int e = 0; e < B * B; e++) v[e] = src[k * (B * B) + e];
-  }
-}
-
+// Refreshes the blob's values from the factor after a numeric factorisation:
+// one thread per packed block (recipe_value, sweep_dev.cuh); D^-1 rows of the
+// forward sweep are copied alongside.
 template <int B, typename TV, bool CPLX>
 __global__ void k_gather_recipes(const ChunkDesc* __restrict__ chunks, unsigned nchunks,
                                  const uint4* __restrict__ recipe, const uint4* __restrict__ terms,
@@ -644,57 +622,13 @@ __global__ void k_gather_recipes(const ChunkDesc* __restrict__ chunks, unsigned 
                                  int with_dinv) {
   static_assert(!CPLX || B == 2, "complex scalars pack as 2x2 blocks");
   constexpr int BB = B * B;
-  constexpr unsigned NONE = 0xffffffffu;
   for (unsigned q = blockIdx.x; q < nchunks; q += gridDim.x) {
     const ChunkDesc cd = chunks[q];
     char* base = blob + cd.off;
     TV* vals = reinterpret_cast<TV*>(base + cd.vals_off);
     for (unsigned k = threadIdx.x; k < cd.nblk_pad; k += blockDim.x) {
-      const uint4 rc = recipe[cd.blk0 + k];
       double v[BB];
-      if (rc.x != NONE) {
-        load_factor_blk<B, CPLX>(foff, rc.x, v);
-      } else {
-#pragma unroll
-        for (int e = 0; e < BB; e++) v[e] = 0.0;
-      }
-      const double sg = rc.w ? -1.0 : 1.0;
-      for (unsigned t = rc.y; t < rc.z; t++) {
-        const uint4 tm = terms[t];
-        double a[BB], m[BB], d[BB];
-        load_factor_blk<B, CPLX>(foff, tm.x, a);
-        if (tm.y != NONE) {  // a = a * D_j^-1
-          load_factor_blk<B, CPLX>(fdiag, tm.y, d);
-#pragma unroll
-          for (int r = 0; r < B; r++)
-#pragma unroll
-            for (int c = 0; c < B; c++) {
-              double acc = 0.0;
-#pragma unroll
-              for (int l = 0; l < B; l++) acc += a[r * B + l] * d[l * B + c];
-              m[r * B + c] = acc;
-            }
-#pragma unroll
-          for (int e = 0; e < BB; e++) a[e] = m[e];
-        }
-        if (tm.z != NONE) {  // a = a * F[s2]
-          double f[BB];
-          load_factor_blk<B, CPLX>(foff, tm.z, f);
-#pragma unroll
-          for (int r = 0; r < B; r++)
-#pragma unroll
-            for (int c = 0; c < B; c++) {
-              double acc = 0.0;
-#pragma unroll
-              for (int l = 0; l < B; l++) acc += a[r * B + l] * f[l * B + c];
-              m[r * B + c] = acc;
-            }
-#pragma unroll
-          for (int e = 0; e < BB; e++) a[e] = m[e];
-        }
-#pragma unroll
-        for (int e = 0; e < BB; e++) v[e] += sg * a[e];
-      }
+      recipe_value<B, CPLX>(recipe[cd.blk0 + k], terms, fdiag, foff, v);
 #pragma unroll
       for (int e = 0; e < BB; e++) vals[(size_t)k * BB + e] = (TV)v[e];
     }
@@ -721,14 +655,18 @@ void sweep_plan_free(SweepPlan* P) {
   cudaFree(P->d_blob);
   cudaFree(P->d_recipe);
   cudaFree(P->d_terms);
+  cudaFree(P->d_ctas);
+  cudaFree(P->d_hchunks);
+  cudaFree(P->d_table);
+  cudaFree(P->d_hids);
   *P = SweepPlan();
 }
 
 int sweep_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, int vec_bytes, SweepPlan* P, bool merge,
-                     bool part, bool halo) {
+                     int part, bool halo, int lpr, int cw) {
   if (halo) {
     if (vec_bytes != 8) return DFM_ERR_UNSUPPORTED;
-    return sweep_halo_plan_build(M, fwd, G, val_bytes, P, part, merge);
+    return sweep_halo_plan_build(M, fwd, G, val_bytes, P, part, merge, lpr, cw);
   }
   const unsigned N = M->N;
   const unsigned b = M->vt == DFM_COMPLEX ? 2u : M->b;  // complex scalars as real 2x2 blocks
@@ -988,6 +926,11 @@ int sweep_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, int vec_bytes, S
 
 int sweep_plan_refresh(dfm_ilu M, SweepPlan* P) {
   if (!P->valid || P->nchunks == 0) { P->stale = false; return DFM_OK; }
+  if (P->halo) {
+    const int rc = sweep_halo_refresh(M, P);
+    if (!rc) P->stale = false;
+    return rc;
+  }
   const int grid = (int)std::min<unsigned>(P->nchunks, (unsigned)M->ctx->nsm * 8);
   const int wd = P->fwd ? 1 : 0;
   cudaStream_t s = M->ctx->stream;

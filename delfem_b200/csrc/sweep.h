@@ -58,6 +58,18 @@ struct ChunkDesc {
   unsigned row0;           // first row of the owning range
 };
 
+// What one CTA of a halo plan works on.
+struct HaloCtaDesc {
+  unsigned chunk0, nchunk, row0, nrow, halo0, nhalo, nround, pad;
+};
+
+// One chunk of a halo plan: its bytes in the blob, rows, and the halo entries needed up to its end.
+struct HaloChunk {
+  unsigned long long off;
+  unsigned bytes, pos0, nrows, need, rec0;
+  unsigned round0, nrounds, table0;  // rounds: of the CTA, count, index in the plan's table
+};
+
 struct SweepPlan {
   bool valid = false;
   bool stale = true;       // values not yet gathered from the current factor
@@ -79,17 +91,26 @@ struct SweepPlan {
   unsigned* d_cta_chunk = nullptr;  // G+1 chunk ranges
   unsigned* d_range = nullptr;      // G+1 ranges of row positions
   unsigned* d_rows = nullptr;       // with a row partition: the row at each position (else positions are rows)
-  bool part = false;                // ranges are the parts of the ILU's row partition
+  int part = 0;                     // 1: ranges are the parts of the ILU's row partition, 2: of its partition by chains
   char* d_blob = nullptr;
   uint4* d_recipe = nullptr;        // per packed block: {base slot, term range, sign}
   uint4* d_terms = nullptr;         // {s1, j, s2, 0}: F[s1] (D_j^-1) (F[s2])
   bool merged = false;              // steps are pairs of levels
-  // halo plans (sweep_halo.cu, schedule mode 9): compute warps read shared memory only
+  // halo plans (sweep_halo.cu, schedule modes 9 and 10): compute warps read shared memory only; lpr lanes per
+  // component of a row, d_rows the rows in the order of every CTA's slice
   bool halo = false;
-  unsigned x_slice = 0;             // elements of the range slice at the start of X
-  unsigned halo_stride = 0;         // elements of one stage's halo area
+  unsigned x_slice = 0;             // elements of the slice (a ring) at the start of X; a zero block follows
+  unsigned halo0 = 0;               // element of the halo area
+  unsigned ring = 0;                // entries of the halo area
+  unsigned rd_off = 0;              // byte offset of the fused dot's vector (0: no room)
+  int parts = 0;                    // parts asked for
+  bool extras = false;              // some rows have more blocks than a lane's registers hold
+  HaloChunk* d_hchunks = nullptr;
+  void* d_table = nullptr;          // rounds, CTA by CTA
+  HaloCtaDesc* d_ctas = nullptr;
+  unsigned* d_hids = nullptr;       // halo rows in the order they are needed, CTA by CTA
   int cw = 4;                       // compute warps
-  int hw = 4;                       // producer warps
+  int hw = 4;                       // halo warps
 };
 
 }  // namespace dfm

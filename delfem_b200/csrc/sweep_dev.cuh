@@ -200,5 +200,78 @@ DFM_DEVINL void st_volatile_s(double* p, double v) { *reinterpret_cast<volatile 
 DFM_DEVINL void st_volatile_s(float* p, float v) { *reinterpret_cast<volatile float*>(p) = v; }
 DFM_DEVINL void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// Values of the packed plans.  Every packed block has a recipe {base, t0, t1, sign}:
+//   value = (base != NONE ? F[base] : 0) + sign * sum_{t0 <= t < t1} F[s1] (D_j^-1) (F[s2])
+// with a term {s1, j, s2} (j or s2 NONE = identity), F the factor's off-diagonal
+// blocks.  Plain operands are copies (no terms); the merged plans' operands of
+// the second level of a pair are the products L_ij D_j^-1 (forward input
+// terms), U'_ij (backward input terms) and the fill blocks
+// F_ik - sum_j F_ij (D_j^-1) F_jk.  CPLX: the factor holds complex scalars
+// (re, im), packed as the real 2x2 blocks [re -im; im re] (B = 2), whose
+// products are the complex products.
+template <int B, bool CPLX>
+DFM_DEVINL void load_factor_blk(const double* __restrict__ src, size_t k, double* v) {
+  if constexpr (CPLX) {
+    const double re = src[2 * k], im = src[2 * k + 1];
+    v[0] = re;
+    v[1] = -im;
+    v[2] = im;
+    v[3] = re;
+  } else {
+#pragma unroll
+    for (int e = 0; e < B * B; e++) v[e] = src[k * (B * B) + e];
+  }
+}
+
+template <int B, bool CPLX>
+DFM_DEVINL void recipe_value(const uint4 rc, const uint4* __restrict__ terms, const double* __restrict__ fdiag,
+                             const double* __restrict__ foff, double* v) {
+  static_assert(!CPLX || B == 2, "complex scalars pack as 2x2 blocks");
+  constexpr int BB = B * B;
+  constexpr unsigned NONE = 0xffffffffu;
+  if (rc.x != NONE) {
+    load_factor_blk<B, CPLX>(foff, rc.x, v);
+  } else {
+#pragma unroll
+    for (int e = 0; e < BB; e++) v[e] = 0.0;
+  }
+  const double sg = rc.w ? -1.0 : 1.0;
+  for (unsigned t = rc.y; t < rc.z; t++) {
+    const uint4 tm = terms[t];
+    double a[BB], m[BB], d[BB];
+    load_factor_blk<B, CPLX>(foff, tm.x, a);
+    if (tm.y != NONE) {  // a = a * D_j^-1
+      load_factor_blk<B, CPLX>(fdiag, tm.y, d);
+#pragma unroll
+      for (int r = 0; r < B; r++)
+#pragma unroll
+        for (int c = 0; c < B; c++) {
+          double acc = 0.0;
+#pragma unroll
+          for (int l = 0; l < B; l++) acc += a[r * B + l] * d[l * B + c];
+          m[r * B + c] = acc;
+        }
+#pragma unroll
+      for (int e = 0; e < BB; e++) a[e] = m[e];
+    }
+    if (tm.z != NONE) {  // a = a * F[s2]
+      double f[BB];
+      load_factor_blk<B, CPLX>(foff, tm.z, f);
+#pragma unroll
+      for (int r = 0; r < B; r++)
+#pragma unroll
+        for (int c = 0; c < B; c++) {
+          double acc = 0.0;
+#pragma unroll
+          for (int l = 0; l < B; l++) acc += a[r * B + l] * f[l * B + c];
+          m[r * B + c] = acc;
+        }
+#pragma unroll
+      for (int e = 0; e < BB; e++) a[e] = m[e];
+    }
+#pragma unroll
+    for (int e = 0; e < BB; e++) v[e] += sg * a[e];
+  }
+}
 
 }  // namespace dfm

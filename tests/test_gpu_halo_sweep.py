@@ -1,0 +1,147 @@
+"""Schedules 9 and 10 at the edges of their packing: rows longer than a lane's
+registers, slices and halo areas kept as rings, a fused dot without room for
+its vector, and partitions by chains.  The preconditioner to 1e-11 of the
+oracle, solves to 1e-8, as in the tests of the other schedules."""
+import numpy as np
+import pytest
+
+from tests import cases
+from oracle import port as P
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a, np.float64)).cuda()
+
+
+def _make(ctx, S):
+    from delfem_b200 import lib
+    A = lib.Matrix(ctx, S.rowptr, S.colind, S.b, lib.COMPLEX if S.cplx else lib.REAL)
+    A.set_values(S.diag, S.off)
+    M = lib.ILU(A)
+    M.factor()
+    return A, M
+
+
+def _apply(M, S, fd, fo, seed=5):
+    r = np.random.default_rng(seed).standard_normal(S.N * S.xw)
+    ref = S.precond(fd, fo, r)
+    z = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+    M.apply(_dev(r), z)
+    assert np.allclose(z.cpu().numpy(), ref, rtol=1e-11, atol=1e-12 * np.abs(ref).max())
+
+
+def _pattern(N, rows, b, seed):
+    """A diagonally dominant system from each row's set of lower columns, made symmetric in pattern."""
+    full = [set() for _ in range(N)]
+    for i, cols in enumerate(rows):
+        for j in cols:
+            full[i].add(j)
+            full[j].add(i)
+    rp = np.concatenate([[0], np.cumsum([len(s) for s in full])]).astype(np.uint32)
+    ci = np.concatenate([np.array(sorted(s), np.uint32) for s in full])
+    S = P.System(rp, ci, b)
+    rng = np.random.default_rng(seed)
+    S.off[:] = rng.uniform(-1.0, 1.0, S.off.size) / (2 * b * max(len(s) for s in full))
+    S.diag[:] = np.tile(np.eye(b).ravel(), N)
+    S.rhs[:] = rng.standard_normal(N * b)
+    return S
+
+
+@pytest.mark.parametrize("b", [1, 2, 3])
+@pytest.mark.parametrize("warps", [(1, 2, 1), (2, 4, 4), (4, 8, 8)])
+@pytest.mark.parametrize("mode", [9, 10])
+@pytest.mark.parametrize("ctas", [1, 5])
+def test_rows_longer_than_the_registers(ctx, b, warps, mode, ctas):
+    """Blocks per lane below, at and far past what a lane holds."""
+    from delfem_b200 import lib
+    S = cases.random_spd_like(220, b, seed=31, density=14)
+    A, M = _make(ctx, S)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+    M.sweep = mode
+    M.sweep_warps = warps
+    _, fd, fo = S.ilu0()
+    _apply(M, S, fd, fo)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+@pytest.mark.parametrize("kind", ["poisson", "solid2d", "solid3d", "helmholtz"])
+@pytest.mark.parametrize("ctas", [1, 6])
+def test_slice_ring_wraps(ctx, kind, ctas):
+    """Parts many times as long as the slice, so its places are taken over; the fused dot follows the ring."""
+    from delfem_b200 import lib
+    S = {"poisson": lambda: cases.poisson(90), "solid2d": lambda: cases.solid2d(60),
+         "solid3d": lambda: cases.solid3d(60, 5, 5), "helmholtz": lambda: cases.helmholtz(30, "bands")}[kind]()[1]
+    A, M = _make(ctx, S)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+    M.sweep = 9
+    _, fd, fo = S.ilu0()
+    _apply(M, S, fd, fo)
+    if kind != "helmholtz":
+        ref = S.solve(fd, fo, tol=1e-10, maxit=2000)
+        x = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+        rc, it, _ = lib.solve_pcg(A, M, _dev(S.rhs), x, tol=1e-10, maxit=2000)
+        assert rc == lib.OK and abs(int(it) - int(ref["iters"])) <= 2
+        assert np.linalg.norm(x.cpu().numpy() - ref["x"]) <= 1e-8 * np.linalg.norm(ref["x"])
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+@pytest.mark.parametrize("b", [1, 3])
+def test_early_rows_read_to_the_end(ctx, b):
+    """The first 64 rows are read by every later row: the slice holds a whole part (12,000 doubles of a
+    part of one CTA leave no room for the dot's vector) and the halo of the other CTAs spans everything."""
+    from delfem_b200 import lib
+    N = 12000 if b == 1 else 4000
+    S = _pattern(N, [{i - 64, i % 64} if i >= 128 else {i - 64} if i >= 64 else set() for i in range(N)], b, 7)
+    A, M = _make(ctx, S)
+    _, fd, fo = S.ilu0()
+    ref = S.solve(fd, fo, tol=1e-10, maxit=500)
+    for ctas in (1, 9):
+        lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+        M.sweep = 9
+        _apply(M, S, fd, fo)
+        x = torch.zeros(S.N * b, dtype=torch.float64, device="cuda")
+        rc, it, _ = lib.solve_pcg(A, M, _dev(S.rhs), x, tol=1e-10, maxit=500)
+        assert rc == lib.OK and abs(int(it) - int(ref["iters"])) <= 1
+        assert np.linalg.norm(x.cpu().numpy() - ref["x"]) <= 1e-8 * np.linalg.norm(ref["x"])
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+def test_halo_ring(ctx):
+    """Every part reads most rows of the others: the halo area (6,000 rows of 24 bytes) is a ring."""
+    from delfem_b200 import lib
+    rng = np.random.default_rng(2)
+    N = 6000
+    S = _pattern(N, [set(rng.integers(0, i, 6).tolist()) if i else set() for i in range(N)], 3, 9)
+    A, M = _make(ctx, S)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 8, 0))
+    M.sweep = 9
+    _, fd, fo = S.ilu0()
+    _apply(M, S, fd, fo)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+@pytest.mark.parametrize("fill", [0, 1])
+def test_partition_by_chains(ctx, fill):
+    """The autotuner's own partitions (chains of a box and of a plane grid) and their PCG."""
+    from delfem_b200 import lib
+    for S in (cases.solid3d(24, 7, 6)[1], cases.poisson(70)[1]):
+        A = lib.Matrix(ctx, S.rowptr, S.colind, S.b)
+        A.set_values(S.diag, S.off)
+        M = lib.ILU(A, fill)
+        M.factor()
+        if fill == 0:
+            _, fd, fo = S.ilu0()
+            _apply(M, S, fd, fo)
+            ref = S.solve(fd, fo, tol=1e-10, maxit=2000)["x"]
+        else:
+            M0 = lib.ILU(A)
+            M0.factor()
+            _, fd, fo = S.ilu0()
+            ref = S.solve(fd, fo, tol=1e-12, maxit=4000)["x"]
+        x = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+        rc, _, _ = lib.solve_pcg(A, M, _dev(S.rhs), x, tol=1e-10, maxit=2000)
+        assert rc == lib.OK
+        assert np.linalg.norm(x.cpu().numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
