@@ -227,6 +227,190 @@ k_ilu0_factor(unsigned N, const unsigned* __restrict__ rowptr, const unsigned* _
   }
 }
 
+// The same factorisation with the row in shared memory, for rows that fit.
+// What bounds it is the chain of levels.  k_ilu0_factor pays a trip through L2
+// per lower block (its column, a search for every target, then the values:
+// ~1,000 cycles each, 7 of them on a tetrahedral mesh), and between two levels
+// a fence, a flag, a poll and another fence; the 200x40x40 box took 4.99 ms
+// for its 281 levels (17.8 us each) beside 0.11 ms of copies.  Here a warp
+// reads its row of A and finds the targets of all updates before it waits, and
+// the U blocks of the rows it reads announce themselves: the factor starts out
+// as a NaN sentinel, so a value that is not one is final, as in the sweeps.
+// They are polled together, and the elimination runs from shared memory.  The
+// operations and their order are the same, so the factor is the same to the
+// bit.
+// Shared memory per warp: ucap U blocks, the row's blocks (the diagonal block
+// last) and columns, where the U blocks come from and go to.
+struct RowFactorShape {
+  unsigned rcap, ucap, vals, cols, from, tgt, warp_bytes;  // blocks; byte offsets
+};
+static RowFactorShape row_factor_shape(unsigned bb, unsigned max_row, unsigned max_up) {
+  RowFactorShape S;
+  S.rcap = max_row + 1;
+  S.ucap = std::max(64u, max_up);
+  S.vals = 8 * bb * S.ucap;                   // U blocks first
+  S.cols = S.vals + 8 * bb * S.rcap;          // then the row
+  S.from = S.cols + 4 * S.rcap;
+  S.tgt = S.from + 4 * S.ucap;
+  S.warp_bytes = (S.tgt + 2 * S.ucap + 15u) & ~15u;
+  return S;
+}
+constexpr unsigned kRowFactorBytes = 24 * 1024;  // per warp, else k_ilu0_factor
+
+// A's values as the factorisation reads them: its own pattern, or (fillmap)
+// the slots of the filled pattern its blocks go to, zero elsewhere.
+struct FactorSource {
+  const double *diag, *off;
+  const unsigned *rowptr, *fillmap;
+};
+
+template <int B, bool CPLX>
+__global__ void __launch_bounds__(256)
+k_ilu_factor_row(unsigned N, FactorSource src, const unsigned* __restrict__ rowptr,
+                 const unsigned* __restrict__ colind, const unsigned* __restrict__ diaind,
+                 const unsigned* __restrict__ order, double* fdiag, double* foff, DevStatus* st, uint64_t wait_ns,
+                 RowFactorShape S) {
+  static_assert(!CPLX || B == 1, "complex blocks are scalars");
+  constexpr unsigned BB = CPLX ? 2 : B * B, FULL = 0xffffffffu;  // doubles per block
+  constexpr unsigned short NOT = 0xffff;
+  extern __shared__ __align__(16) char fsmem[];
+  const unsigned lane = threadIdx.x & 31u;
+  char* mine = fsmem + (threadIdx.x >> 5) * S.warp_bytes;
+  double* uv = reinterpret_cast<double*>(mine);
+  double* rv = reinterpret_cast<double*>(mine + S.vals);
+  unsigned* rc = reinterpret_cast<unsigned*>(mine + S.cols);
+  unsigned* from = reinterpret_cast<unsigned*>(mine + S.from);
+  unsigned short* tgt = reinterpret_cast<unsigned short*>(mine + S.tgt);
+  const unsigned w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  // entry el of the product of the blocks l and u, as the reference sums it
+  auto product = [](const double* l, const double* u, unsigned el) {
+    if constexpr (CPLX) {
+      return el ? add_rn(mul_rn(l[0], u[1]), mul_rn(l[1], u[0])) : sub_rn(mul_rn(l[0], u[0]), mul_rn(l[1], u[1]));
+    } else {
+      const unsigned r = el / B, c = el - r * B;
+      double acc = mul_rn(l[r * B], u[c]);
+#pragma unroll
+      for (int m = 1; m < B; m++) acc = add_rn(acc, mul_rn(l[r * B + m], u[m * B + c]));
+      return acc;
+    }
+  };
+  for (unsigned p = w0; p < N; p += nw) {
+    const unsigned i = __ldg(order + p);
+    const unsigned s0 = __ldg(rowptr + i), s1 = __ldg(rowptr + i + 1), di = __ldg(diaind + i);
+    const unsigned nnz = s1 - s0, nl = di - s0;
+    for (unsigned q = lane; q < nnz; q += 32) rc[q] = __ldg(colind + s0 + q);
+    if (src.fillmap) {
+      for (unsigned q = lane; q < nnz * BB; q += 32) rv[q] = 0.0;
+      __syncwarp();
+      const unsigned a0 = __ldg(src.rowptr + i), na = __ldg(src.rowptr + i + 1) - a0;
+      for (unsigned q = lane; q < na * BB; q += 32)
+        rv[(__ldg(src.fillmap + a0 + q / BB) - s0) * BB + q % BB] = __ldcs(src.off + (size_t)a0 * BB + q);
+    } else {
+      for (unsigned q = lane; q < nnz * BB; q += 32) rv[q] = __ldcs(src.off + (size_t)s0 * BB + q);
+    }
+    if (lane < BB) rv[nnz * BB + lane] = __ldcs(src.diag + (size_t)i * BB + lane);
+    __syncwarp();
+    double* d = rv + nnz * BB;
+    for (unsigned e0 = 0; e0 < nl;) {
+      // the next lower blocks whose rows' U blocks fit together: lane l has block e0 + l
+      unsigned u0 = 0, len = 0;
+      if (e0 + lane < nl) {
+        const unsigned k = rc[e0 + lane];
+        u0 = __ldg(diaind + k);
+        len = __ldg(rowptr + k + 1) - u0;
+      }
+      unsigned end = len;  // inclusive prefix sum: where the lane's U blocks end
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(FULL, end, o);
+        if (lane >= (unsigned)o) end += t;
+      }
+      const unsigned ne = (unsigned)__popc(__ballot_sync(FULL, e0 + lane < nl && end <= S.ucap));  // >= 1
+      // targets of their blocks in this row (no fill-in beyond the pattern)
+      for (unsigned e = 0; e < ne; e++) {
+        const unsigned ue = __shfl_sync(FULL, u0, (int)e), n = __shfl_sync(FULL, len, (int)e);
+        const unsigned at = __shfl_sync(FULL, end, (int)e) - n;
+        for (unsigned b = lane; b < n; b += 32) {
+          const unsigned j = __ldg(colind + ue + b);
+          unsigned lo = 0, hi = nnz;
+          while (lo < hi) {
+            const unsigned m = (lo + hi) >> 1;
+            if (rc[m] < j) lo = m + 1; else hi = m;
+          }
+          tgt[at + b] = j == i ? (unsigned short)nnz : lo < nnz && rc[lo] == j ? (unsigned short)lo : NOT;
+          from[at + b] = ue + b;
+        }
+      }
+      __syncwarp();
+      const unsigned total = __shfl_sync(FULL, end, (int)ne - 1) * BB;
+      // wait for the last value of each row's U blocks, then read them all (again while one is missing)
+      {
+        const double* last = lane < ne && len ? foff + (size_t)(u0 + len) * BB - 1 : nullptr;
+        SpinGuard g(wait_ns);
+        bool miss = __any_sync(FULL, last && Sent<double>::is(ld_relaxed(last)));
+        for (;;) {
+          if (!miss) {
+            bool m = false;
+#pragma unroll 8
+            for (unsigned q = lane; q < total; q += 32) {  // all in flight together
+              const double v = ld_relaxed(foff + (size_t)from[q / BB] * BB + q % BB);
+              m |= Sent<double>::is(v);
+              uv[q] = v;
+            }
+            if (!__any_sync(FULL, m)) break;
+          }
+          if (g.expired() || ((g.n & 1023u) == 0 && ld_status(st) != 0)) {
+            raise_error(st, DFM_WAIT_TIMEOUT, 1);
+            break;
+          }
+          miss = __any_sync(FULL, last && Sent<double>::is(ld_relaxed(last)));
+        }
+      }
+      __syncwarp();
+      for (unsigned e = 0; e < ne; e++) {  // k ascending
+        const unsigned n = __shfl_sync(FULL, len, (int)e), at = __shfl_sync(FULL, end, (int)e) - n;
+        const double* l = rv + (e0 + e) * BB;
+        for (unsigned q = lane; q < n * BB; q += 32) {
+          const unsigned b = q / BB, el = q - b * BB;
+          const unsigned t = tgt[at + b];
+          if (t == NOT) continue;
+          rv[t * BB + el] = sub_rn(rv[t * BB + el], product(l, uv + (at + b) * BB, el));
+        }
+        __syncwarp();
+      }
+      e0 += ne;
+    }
+    // every lane inverts the pivot
+    double a[BB];
+#pragma unroll
+    for (unsigned q = 0; q < BB; q++) a[q] = d[q];
+    bool sing;
+    if constexpr (CPLX) {
+      const double n2 = add_rn(mul_rn(a[0], a[0]), mul_rn(a[1], a[1]));
+      sing = n2 < 1.0e-20;  // the reference stops for a key press here
+      const double fact = __ddiv_rn(1.0, n2);
+      a[0] = mul_rn(fact, a[0]);
+      a[1] = mul_rn(-fact, a[1]);
+    } else {
+      sing = !invert_pivot<B>(a);
+    }
+    if (lane == 0 && sing) atomicAdd(&st->nsing, 1u);
+    __syncwarp();
+    if (lane == 0)
+#pragma unroll
+      for (unsigned q = 0; q < BB; q++) d[q] = a[q];
+    __syncwarp();
+    // U first: others wait for it
+    for (unsigned q = nl * BB + lane; q < nnz * BB; q += 32) {
+      const unsigned b = q / BB, el = q - b * BB;
+      st_relaxed(foff + (size_t)s0 * BB + q, CPLX ? product(rv + b * BB, d, el) : product(d, rv + b * BB, el));
+    }
+    for (unsigned q = lane; q < nl * BB; q += 32) __stcg(foff + (size_t)s0 * BB + q, rv[q]);
+    if (lane < BB) __stcg(fdiag + (size_t)i * BB + lane, d[lane]);
+    __syncwarp();  // the next row overwrites this one's shared memory
+  }
+}
+
 // complex b = 1 (CZMatDiaFrac_BlkCrs::DoILUDecomp)
 DFM_DEVINL double2 zmul_rn(double2 a, double2 b) {
   return make_double2(sub_rn(mul_rn(a.x, b.x), mul_rn(a.y, b.y)), add_rn(mul_rn(a.x, b.y), mul_rn(a.y, b.x)));
@@ -589,19 +773,21 @@ __global__ void k_wait_selftest(const double* never, DevStatus* st, uint64_t wai
 }
 
 // ---------------------------------------------------------------- launches
-static int coop_grid(const void* fn, int threads, int nsm, int cap) {
+static int coop_grid(const void* fn, int threads, int nsm, int cap, size_t smem = 0) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0) != cudaSuccess) return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) return -1;
   per_sm = std::max(1, std::min(per_sm, 8));
   return std::max(1, std::min(per_sm * nsm, cap));
 }
 
 // Co-resident persistent launch (cooperative attribute: all blocks resident).
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_coop(void (*fn)(KArgs...), int grid, int threads, cudaStream_t s, Args... args) {
+static cudaError_t launch_coop_smem(void (*fn)(KArgs...), int grid, int threads, size_t smem, cudaStream_t s,
+                                    Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -610,17 +796,39 @@ static cudaError_t launch_coop(void (*fn)(KArgs...), int grid, int threads, cuda
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, fn, static_cast<KArgs>(args)...);
 }
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_coop(void (*fn)(KArgs...), int grid, int threads, cudaStream_t s, Args... args) {
+  return launch_coop_smem(fn, grid, threads, 0, s, args...);
+}
+
+// CTAs of the factorisation, 8 rows at a time each: a few levels' rows in flight.  More would only poll rows that are
+// levels away.
+static int factor_ctas(dfm_ilu M) {
+  const unsigned rows = std::min(M->N, 12 * (M->N / std::max(1u, M->nlev_f) + 1));
+  return (int)((rows + 7) / 8);
+}
 
 int ilu_factor_launch(dfm_ilu M, dfm_mat A) {
   dfm_ctx c = M->ctx;
   cudaStream_t s = c->stream;
   const size_t vw = M->vw();
-  DFM_CUDA_TRY(cudaMemcpyAsync(M->d_fdiag, A->d_diag, sizeof(double) * vw * M->N, cudaMemcpyDeviceToDevice, s));
-  if (M->d_fillmap) {  // ILU(k): A's blocks into the filled pattern, zero elsewhere (SetValue_Initialize)
-    const int rc = ilu_fill_values(M, A);
+  if (M->max_up == ~0u) {
+    M->max_up = 0;
+    for (unsigned i = 0; i < M->N; i++) M->max_up = std::max(M->max_up, M->A->h_rowptr[i + 1] - M->h_diaind[i]);
+  }
+  const RowFactorShape S = row_factor_shape((unsigned)vw, M->A->max_row, M->max_up);
+  const bool rows_fit = S.warp_bytes <= kRowFactorBytes && S.rcap < 0xffffu;
+  if (rows_fit) {  // reads A itself; the factor starts out as the sentinel
+    const int rc = ilu_fill_sentinel(M, M->d_foff, vw * M->ncrs);
     if (rc) return rc;
-  } else if (M->ncrs) {
-    DFM_CUDA_TRY(cudaMemcpyAsync(M->d_foff, A->d_off, sizeof(double) * vw * M->ncrs, cudaMemcpyDeviceToDevice, s));
+  } else {
+    DFM_CUDA_TRY(cudaMemcpyAsync(M->d_fdiag, A->d_diag, sizeof(double) * vw * M->N, cudaMemcpyDeviceToDevice, s));
+    if (M->d_fillmap) {  // ILU(k): A's blocks into the filled pattern, zero elsewhere (SetValue_Initialize)
+      const int rc = ilu_fill_values(M, A);
+      if (rc) return rc;
+    } else if (M->ncrs) {
+      DFM_CUDA_TRY(cudaMemcpyAsync(M->d_foff, A->d_off, sizeof(double) * vw * M->ncrs, cudaMemcpyDeviceToDevice, s));
+    }
   }
   DFM_CUDA_TRY(cudaMemsetAsync(&c->d_status->nsing, 0, sizeof(unsigned), s));
   M->plan_f.stale = true;  // packed sweep values are re-gathered on next use
@@ -633,8 +841,20 @@ int ilu_factor_launch(dfm_ilu M, dfm_mat A) {
     M->epoch = 1;
   }
   if (M->N == 0) return DFM_OK;
-  cudaError_t e;
-  if (M->vt == DFM_COMPLEX) {
+  cudaError_t e = cudaSuccess;
+  const FactorSource src = {A->d_diag, A->d_off, M->user->d_rowptr, M->d_fillmap};
+  const int rsmem = (int)(8 * S.warp_bytes);
+  auto by_rows = [&](auto fn) {
+    cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, rsmem);
+    if (err != cudaSuccess) return err;
+    const int grid = coop_grid((const void*)fn, 256, c->nsm, factor_ctas(M), rsmem);
+    return launch_coop_smem(fn, grid, 256, rsmem, s, M->N, src, (const unsigned*)M->A->d_rowptr,
+                            (const unsigned*)M->A->d_colind, (const unsigned*)M->d_diaind,
+                            (const unsigned*)M->d_order_f, M->d_fdiag, M->d_foff, c->d_status, (uint64_t)c->wait_ns, S);
+  };
+  if (M->vt == DFM_COMPLEX && rows_fit) {
+    e = by_rows(k_ilu_factor_row<1, true>);
+  } else if (M->vt == DFM_COMPLEX) {
     const int grid = coop_grid((const void*)k_zilu0_factor, 256, c->nsm, (M->N + 7) / 8);
     e = launch_coop(k_zilu0_factor, grid, 256, s, M->N, (const unsigned*)M->A->d_rowptr,
                     (const unsigned*)M->A->d_colind, (const unsigned*)M->d_diaind, (const unsigned*)M->d_order_f,
@@ -643,6 +863,10 @@ int ilu_factor_launch(dfm_ilu M, dfm_mat A) {
   } else {
 #define DFM_ILU_CASE(BV)                                                                                      \
   case BV: {                                                                                                  \
+    if (rows_fit) {                                                                                           \
+      e = by_rows(k_ilu_factor_row<BV, false>);                                                               \
+      break;                                                                                                  \
+    }                                                                                                         \
     const int grid = coop_grid((const void*)k_ilu0_factor<BV>, 256, c->nsm, (M->N + 7) / 8);                  \
     e = launch_coop(k_ilu0_factor<BV>, grid, 256, s, M->N, (const unsigned*)M->A->d_rowptr,                   \
                     (const unsigned*)M->A->d_colind, (const unsigned*)M->d_diaind,                           \
