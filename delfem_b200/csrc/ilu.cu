@@ -1130,15 +1130,15 @@ int ilu_autotune(dfm_ilu M) {
     Cand top = {0, 0, 0, 0, false};
     float top_ms = 1e30f;
     int err = DFM_OK;
-    // builds and times a candidate; false if it cannot be built
-    auto eval = [&](const Cand& c) {
+    // builds and times a candidate: its ms, or 1e30 if it cannot be built
+    auto eval = [&](const Cand& c) -> float {
       SweepPlan pf, pb;
       if (sweep_plan_build(M, true, c.G, 8, 8, &pf, c.merge, c.part, true, c.lpr, c.cw) != DFM_OK ||
           sweep_plan_build(M, false, c.G, 8, 8, &pb, c.merge, c.part, true, c.lpr, c.cw) != DFM_OK) {
         sweep_plan_free(&pf);
         sweep_plan_free(&pb);
         cudaGetLastError();
-        return;
+        return 1e30f;
       }
       pf.hw = pb.hw = 9 - c.cw;  // every warp the launch has left polls halo rows
       std::swap(M->plan_f, pf);  // M holds the candidate
@@ -1156,6 +1156,7 @@ int ilu_autotune(dfm_ilu M) {
       }
       sweep_plan_free(&pf);
       sweep_plan_free(&pb);
+      return rc == DFM_OK ? ms : 1e30f;
     };
     // rows whose blocks do not fit the lanes' registers take the slower kernel for longer rows
     unsigned long_rows = 0;
@@ -1171,17 +1172,22 @@ int ilu_autotune(dfm_ilu M) {
     };
     const bool large = M->N > 150000;  // a plan takes tenths of a second there
     if (M->nparts > 0 && M->nparts <= (unsigned)nsm) eval({1, (int)M->nparts, h0, warps_for((int)M->nparts), false});
-    const int counts[] = {nsm, 64, 32, 24, 16, 12, 8, 6, 4, 2, 1};
-    float last = 1e30f;
-    int worse = 0;
-    for (int G : counts) {
-      if (err || worse > 1 || (large && G < 64)) break;
-      if (G > nsm || (G > 1 && M->N < 64u * (unsigned)G)) continue;
-      const float before = top_ms;
-      eval({2, G, h0, warps_for(G), false});
-      if (!large || G == nsm) eval({0, G, h0, warps_for(G), false});
-      worse = before < 1e29f && top_ms == before && last < 1e29f ? worse + 1 : 0;
-      last = top_ms;
+    // parts by chains or ranges of the natural order, compared at a middle count; then more and fewer CTAs with the
+    // better of the two while they get faster (fewer CTAs: shorter chains of hand-overs; more: shorter rounds)
+    auto allowed = [&](int G) { return G <= nsm && (G == 1 || M->N >= 64u * (unsigned)G); };
+    const int first = large ? nsm : M->N >= 64u * 16u ? 16 : 1;
+    const float by_chains = err ? 1e30f : eval({2, first, h0, warps_for(first), false});
+    const float by_ranges = err ? 1e30f : eval({0, first, h0, warps_for(first), false});
+    const int kind = by_chains <= by_ranges ? 2 : 0;
+    for (const std::initializer_list<int>& side : {std::initializer_list<int>{32, 64, nsm}, {12, 8, 4, 2, 1}}) {
+      float last = std::min(by_chains, by_ranges);
+      for (int G : side) {
+        if (err || large || first == 1) break;
+        if (!allowed(G)) continue;
+        const float ms = eval({kind, G, h0, warps_for(G), false});
+        if (ms > last && last < 1e29f) break;
+        last = ms;
+      }
     }
     if (top.G) {
       Cand c = top;
@@ -1197,10 +1203,10 @@ int ilu_autotune(dfm_ilu M) {
         d.cw = d.lpr > top.lpr ? std::min(4, 2 * top.cw) : std::max(1, top.cw / 2);
         eval(d);
       }
-      if (!err && !large) {
+      if (!err && !large && bx < 3) {
         Cand d = top;
         d.merge = true;
-        if (bx < 3) d.lpr = 2;  // a merged row has about twice the blocks
+        d.lpr = 2;  // a merged row has about twice the blocks
         eval(d);
       }
     }

@@ -648,17 +648,17 @@ __global__ void k_gather_recipes(const ChunkDesc* __restrict__ chunks, unsigned 
 // ------------------------------------------------------------- host plan
 void sweep_plan_free(SweepPlan* P) {
   if (!P) return;
-  cudaFree(P->d_chunks);
-  cudaFree(P->d_cta_chunk);
-  cudaFree(P->d_range);
-  cudaFree(P->d_rows);
-  cudaFree(P->d_blob);
-  cudaFree(P->d_recipe);
-  cudaFree(P->d_terms);
-  cudaFree(P->d_ctas);
-  cudaFree(P->d_hchunks);
-  cudaFree(P->d_table);
-  cudaFree(P->d_hids);
+  if (P->d_arena) {
+    cudaFree(P->d_arena);
+  } else {
+    cudaFree(P->d_chunks);
+    cudaFree(P->d_cta_chunk);
+    cudaFree(P->d_range);
+    cudaFree(P->d_rows);
+    cudaFree(P->d_blob);
+    cudaFree(P->d_recipe);
+    cudaFree(P->d_terms);
+  }
   *P = SweepPlan();
 }
 

@@ -99,6 +99,7 @@ struct SweepPlan {
   // halo plans (sweep_halo.cu, schedule modes 9 and 10): compute warps read shared memory only; lpr lanes per
   // component of a row, d_rows the rows in the order of every CTA's slice
   bool halo = false;
+  char* d_arena = nullptr;          // the one allocation all of a halo plan's arrays are in
   unsigned x_slice = 0;             // elements of the slice (a ring) at the start of X; a zero block follows
   unsigned halo0 = 0;               // element of the halo area
   unsigned ring = 0;                // entries of the halo area

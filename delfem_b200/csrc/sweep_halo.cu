@@ -77,13 +77,15 @@ constexpr int kHaloRhsWarps = 2;
 constexpr int kHaloMaxWarps = 12;  // compute, copy, right-hand-side and halo warps of a launch
 constexpr int kHaloMaxThreads = 32 * kHaloMaxWarps;
 constexpr int kHaloMaxCw = 4;
-constexpr unsigned kHaloChunkBytes = 12 * 1024;  // a chunk closes past this
+// A chunk closes when a round like its last would take it past kHaloChunkBytes.  Taking a chunk over costs the compute
+// warps some 300 cycles, so chunks hold several rounds as long as enough stages fit.
+constexpr unsigned kHaloChunkBytes = 24 * 1024;
 constexpr unsigned kHaloReuse = 8;  // chunks after its own that may read an entry of a halo ring
 constexpr size_t kHaloSmemBudget = 220 * 1024;  // dynamic shared memory per CTA
-// A chunk is entered when its last round's look-ahead (two rounds further) is in, and its predecessor's stage is freed
-// then: five chunks must fit so that this waits for no copy that was only just requested.
+// A chunk is entered when the two after it are in, and its predecessor's stage is freed then: five chunks must fit so
+// that this waits for no copy that was only just requested.
 constexpr int kHaloMinStages = 5;
-constexpr int kHaloGoodStages = 8;  // enough to cover a copy's latency
+constexpr int kHaloGoodStages = 6;  // enough to cover a copy's latency
 constexpr unsigned kHaloChunkRounds = 31;  // and at this many rounds
 constexpr unsigned kHaloTable = 512;       // entries of the round-table ring: the rounds of more than kHaloMaxStages chunks
 static_assert(kHaloTable > kHaloChunkRounds * (kHaloMaxStages + 2) && (kHaloTable & (kHaloTable - 1)) == 0, "table ring");
@@ -91,11 +93,12 @@ static_assert(kHaloTable > kHaloChunkRounds * (kHaloMaxStages + 2) && (kHaloTabl
 // A chunk: [row indices u32, padded to 16 bytes][records per round].
 // A record: [K operand offsets u32][K x B values][D^-1 row (forward)][extra blocks: offsets | values].
 // A round's table entry: rec, rows: byte offsets in shared memory of its records and row indices; slot: byte
-// offset in X of its first row; shape: rows | pieces of a record << 8 | extra blocks per lane << 20.
+// offset in X of its first row; shape: rows | pieces of a record << 8 | extra blocks per lane << 20 | last round of
+// its chunk << 31.
 struct HaloRound {
   unsigned rec, slot, rows, shape;
 };
-constexpr unsigned kHaloMaxPieces = 0xfff;
+constexpr unsigned kHaloMaxPieces = 0xfff, kHaloMaxExtra = 0x7ff, kHaloLast = 0x80000000u;
 
 // Record layout of B x B blocks with KT blocks per lane in registers.
 template <int B, int KT, typename TV, bool FWD>
@@ -182,7 +185,7 @@ struct LaneItem {
   unsigned o[R::PO * 4];
   unsigned w[R::PV * 4];
   unsigned row, slot;  // the row's index in the vectors, its component's offset in X
-  bool act;            // the lane has a row
+  bool act, last;      // the lane has a row; the round is its chunk's last
   unsigned extra, rec; // extra blocks per lane, the record's offset (EX only)
   DFM_DEVINL double val(int i) const {
     if constexpr (sizeof(TV) == 8) return __hiloint2double((int)w[2 * i + 1], (int)w[2 * i]);
@@ -210,10 +213,11 @@ DFM_DEVINL void item_load(LaneItem<B, KT, TV, FWD>& P, const char* smem, const u
                           unsigned wrap) {
   using R = HaloRec<B, KT, TV, FWD>;
   P.act = rw < (e.w & 0xffu);
+  P.last = (e.w & kHaloLast) != 0;
   const unsigned r = P.act ? rw : 0u, l = P.act ? rw * (B * H) + idx : 0u;
   unsigned rec;
   if (EX) {
-    P.extra = e.w >> 20;
+    P.extra = (e.w >> 20) & kHaloMaxExtra;
     rec = e.x + l * (16u * ((e.w >> 8) & kHaloMaxPieces));
     P.rec = rec;
   } else {
@@ -311,25 +315,17 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
     const unsigned rw = wl < RPW * LR ? (unsigned)warp * RPW + wl / LR : 0xffffu;  // the lane's row of a round
     const bool writes = idx < B;
     double* outc = out + idx % B;
-    const HaloChunk* my_chunks = chunks + me.chunk0;
-    auto rounds_of = [&](unsigned k) { return k + wl < K ? my_chunks[k + wl].nrounds : 0u; };
-    unsigned cn = rounds_of(0), fn = cn;  // rounds of chunks 32 i + lane, for the two positions below
-    unsigned ck = 0, ck_end = 0, ck_s = 0, ck_par = 0;  // chunks that have landed, the rounds they cover
-    unsigned fr = 0, fr_s = 0;  // the chunk in work
-    unsigned q = 0, mark = 0;   // the round, the first round of the next chunk
+    unsigned k = 0, s = 0;       // the chunk in work, its stage
+    unsigned ls = 0, lpar = 0;   // the stage and its phase of the next chunk to wait for
+    unsigned q = 0;              // the round
     I P0, P1;
     uint4 e1 = make_uint4(0, 0, 0, 0);
-    // landed chunks cover the rounds below r
-    auto cover = [&](unsigned r) {
-      bool ok = true;
-      while (ok && ck_end < r && ck < K) {
-        ok = __all_sync(FULL, spin_until([&] { return mbar_test(&landed[ck_s], ck_par); }, &s_alive, st, wait_ns, 21));
-        ck_end += __shfl_sync(FULL, cn, (int)(ck & 31u));
-        if ((++ck & 31u) == 0) cn = rounds_of(ck);
-        if (++ck_s == ns) {
-          ck_s = 0;
-          ck_par ^= 1u;
-        }
+    auto await_chunk = [&] {
+      const bool ok =
+          __all_sync(FULL, spin_until([&] { return mbar_test(&landed[ls], lpar); }, &s_alive, st, wait_ns, 21));
+      if (++ls == ns) {
+        ls = 0;
+        lpar ^= 1u;
       }
       return ok;
     };
@@ -342,20 +338,19 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
           m |= halo_missing<B>(smem, reinterpret_cast<const unsigned*>(smem + P.rec + 16 * R::P)[k]);
       return m;
     };
-    // before round q, whose item is P: a new chunk, its operands; false to stop
-    auto event = [&](const I& P) {
+    // Before round q, whose item is P: its operands; after the last round of a chunk (last) its stage is handed back
+    // and the chunk after the next waited for: the last round of the next one reads a record and a table entry ahead,
+    // which are in those two.  False to stop.
+    auto event = [&](const I& P, bool last) {
       bool ok = true;
-      if (q == mark) {
-        if (q == me.nround) return false;
-        if (q > 0) {  // round q - 1 was the last of its chunk
-          if (threadIdx.x == 0) mbar_arrive(&free_[fr_s]);
-          if (++fr_s == ns) fr_s = 0;
-          if ((++fr & 31u) == 0) fn = rounds_of(fr);
-        }
-        mark += __shfl_sync(FULL, fn, (int)(fr & 31u));
-        ok = cover(mark + 2);  // the chunk's last round reads the record and the table entry ahead
+      if (last) {
+        if (threadIdx.x == 0) mbar_arrive(&free_[s]);
+        if (++s == ns) s = 0;
+        if (++k == K) return false;
+        if (k + 2 < K) ok = await_chunk();
       }
-      if (ok) ok = __all_sync(FULL, spin_until([&] { return !__any_sync(FULL, missing(P)); }, &s_alive, st, wait_ns, 23));
+      if (ok && __any_sync(FULL, missing(P)))
+        ok = __all_sync(FULL, spin_until([&] { return !__any_sync(FULL, missing(P)); }, &s_alive, st, wait_ns, 23));
       __threadfence_block();
       return ok;
     };
@@ -401,21 +396,22 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
           dim += idx ? r.x * v : r.y * v;
         }
       }
-      const bool ev = __any_sync(FULL, missing(N)) || q + 1 == mark;
+      const bool ev = __any_sync(FULL, missing(N)) || C.last;
       meet(ncw);
       q++;
       return ev;
     };
-    bool go = me.nround > 0 && cover(2);
+    bool go = K > 0;
+    for (unsigned j = 0; j < 3 && j < K && go; j++) go = await_chunk();
     if (go) {
       e1 = *reinterpret_cast<const uint4*>(tab);
       item_load<B, H, KT, TV, FWD, EX>(P0, smem, e1, rw, idx, wrap);
       e1 = *reinterpret_cast<const uint4*>(tab + 1);
-      go = event(P0);
+      go = event(P0, false);
     }
     while (go) {
-      if (body(P0, P1) && !event(P1)) break;
-      if (body(P1, P0) && !event(P0)) break;
+      if (body(P0, P1) && !event(P1, P0.last)) break;
+      if (body(P1, P0) && !event(P0, P1.last)) break;
     }
     // every compute warp passes every round's barrier, stopped or not
     for (; q < me.nround; q++) meet(ncw);
@@ -616,7 +612,7 @@ __global__ void k_gather_halo(const HaloChunk* __restrict__ chunks, unsigned nch
     char* recs = base + cl_al16(4 * cd.nrows);
     for (unsigned j = 0; j < cd.nrounds; j++) {
       const unsigned shape = table[cd.table0 + j].shape;
-      const unsigned n = shape & 0xffu, pieces = (shape >> 8) & kHaloMaxPieces, ke = shape >> 20;
+      const unsigned n = shape & 0xffu, pieces = (shape >> 8) & kHaloMaxPieces, ke = (shape >> 20) & kHaloMaxExtra;
       const unsigned nb = (KT + ke) * uH;  // packed blocks per row
       for (unsigned t = threadIdx.x; t < n * nb; t += blockDim.x) {
         const uint4 rc = recipe[rec0 + t];
@@ -897,13 +893,14 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
           C.extras = C.extras || ke;
           at += 16u * pieces * rd.nrow * S.B * S.H;
         }
-        cd.bytes = at;
+        tab[nround - 1].shape |= kHaloLast;
+      cd.bytes = at;
         C.blob.resize(C.blob.size() + at, 0);
         char* base = C.blob.data() + cd.off;
         std::memcpy(base, C.rows.data() + pos0, 4 * (size_t)nrow);
         for (unsigned j = 0; j < nround; j++) {
           const Round& rd = rounds[j];
-          const unsigned ke = tab[j].shape >> 20, pieces = (tab[j].shape >> 8) & kHaloMaxPieces;
+          const unsigned ke = (tab[j].shape >> 20) & kHaloMaxExtra, pieces = (tab[j].shape >> 8) & kHaloMaxPieces;
           const unsigned nb = (S.KT + ke) * S.H;
           for (unsigned r = 0; r < rd.nrow; r++) {
             const unsigned q0 = op0[rd.row0 + r], q1 = op0[rd.row0 + r + 1];
@@ -970,10 +967,11 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
           rd.nrow++;
         }
         const unsigned ke = rd.K > S.KT ? rd.K - S.KT : 0u;
-        if (ke > 0xfffu || S.pieces(ke) > kHaloMaxPieces) return DFM_ERR_UNSUPPORTED;
+        if (ke > kHaloMaxExtra || S.pieces(ke) > kHaloMaxPieces) return DFM_ERR_UNSUPPORTED;
         rounds.push_back(rd);
-        bytes += 16u * S.pieces(ke) * rd.nrow * S.B * S.H + 4u * rd.nrow;
-        if (bytes >= chunk_bytes || rounds.size() == kHaloChunkRounds || p == todo.size()) {
+        const unsigned more = 16u * S.pieces(ke) * rd.nrow * S.B * S.H + 4u * rd.nrow;
+        bytes += more;
+        if (bytes + more > chunk_bytes || rounds.size() == kHaloChunkRounds || p == todo.size()) {
           close();
           bytes = 0;
         }
@@ -1097,7 +1095,7 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
       const unsigned stage = (unsigned)(x_bytes + (q % (size_t)ns) * stage_max);
       for (unsigned j = 0; j < cd.nrounds; j++) {
         HaloRound& rd = C.table[cd.round0 + j];
-        const unsigned ke = rd.shape >> 20, pieces = (rd.shape >> 8) & kHaloMaxPieces;
+        const unsigned ke = (rd.shape >> 20) & kHaloMaxExtra, pieces = (rd.shape >> 8) & kHaloMaxPieces;
         const unsigned nrec_j = (rd.shape & 0xffu) * S.B * S.H;
         for (unsigned l = 0; l < nrec_j; l++) {
           char* rec = base + rd.rec + 16 * (size_t)pieces * l;
@@ -1121,7 +1119,7 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
     }
     if (!C.table.empty()) {  // past the last round: its records, no rows
       C.table.push_back(C.table.back());
-      C.table.back().shape &= ~0xffu;
+      C.table.back().shape &= ~(0xffu | kHaloLast);
     }
     for (uint4& r : C.recipe) {
       r.y += (unsigned)term0;
@@ -1152,34 +1150,54 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
   P->cw = cw;
   P->hw = 4;
   cudaStream_t s = M->ctx->stream;
-  DFM_CUDA_TRY(cudaMalloc(&P->d_hchunks, sizeof(HaloChunk) * std::max<size_t>(chunks.size(), 1)));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_ctas, sizeof(HaloCtaDesc) * G));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_table, sizeof(HaloRound) * std::max<size_t>(nround, 1)));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_rows, sizeof(unsigned) * std::max(N, 1u)));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_hids, sizeof(unsigned) * std::max<size_t>(nhid, 1)));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_blob, std::max<size_t>(blob_size, 16)));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_recipe, sizeof(uint4) * std::max<size_t>(nrec, 1)));
-  DFM_CUDA_TRY(cudaMalloc(&P->d_terms, sizeof(uint4) * std::max<size_t>(nterm, 1)));
-  auto put = [&](void* dst, const void* src, size_t bytes) {
-    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
+  // one allocation: the blob, then the arrays (16-byte aligned); the arrays go over in one copy from `host`, the blob
+  // CTA by CTA
+  size_t at = (blob_size + 255) & ~(size_t)255;
+  const size_t arrays0 = at;
+  auto place = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 15) & ~(size_t)15;
+    return o;
   };
+  const size_t o_chunks = place(sizeof(HaloChunk) * chunks.size()), o_ctas = place(sizeof(HaloCtaDesc) * G);
+  const size_t o_table = place(sizeof(HaloRound) * nround), o_rows = place(sizeof(unsigned) * N);
+  const size_t o_hids = place(sizeof(unsigned) * nhid), o_rec = place(sizeof(uint4) * nrec);
+  const size_t o_terms = place(sizeof(uint4) * nterm);
+  std::vector<char> host(at - arrays0 + 16);
+  auto put = [&](size_t o, const void* src, size_t bytes) {
+    if (bytes) std::memcpy(host.data() + (o - arrays0), src, bytes);
+  };
+  put(o_chunks, chunks.data(), sizeof(HaloChunk) * chunks.size());
+  put(o_ctas, desc.data(), sizeof(HaloCtaDesc) * G);
   rec0 = term0 = off0 = hid0 = tab0 = 0;
   for (int c = 0; c < G; c++) {
     const HaloCta& C = ctas[c];
-    DFM_CUDA_TRY(put(P->d_blob + off0, C.blob.data(), C.blob.size()));
-    DFM_CUDA_TRY(put(P->d_recipe + rec0, C.recipe.data(), sizeof(uint4) * C.recipe.size()));
-    DFM_CUDA_TRY(put(P->d_terms + term0, C.terms.data(), sizeof(uint4) * C.terms.size()));
-    DFM_CUDA_TRY(put(P->d_hids + hid0, C.hids.data(), sizeof(unsigned) * C.hids.size()));
-    DFM_CUDA_TRY(put(reinterpret_cast<HaloRound*>(P->d_table) + tab0, C.table.data(), sizeof(HaloRound) * C.table.size()));
-    tab0 += C.table.size();
-    DFM_CUDA_TRY(put(P->d_rows + range[c], C.rows.data(), sizeof(unsigned) * C.rows.size()));
-    off0 += C.blob.size();
+    put(o_rec + sizeof(uint4) * rec0, C.recipe.data(), sizeof(uint4) * C.recipe.size());
+    put(o_terms + sizeof(uint4) * term0, C.terms.data(), sizeof(uint4) * C.terms.size());
+    put(o_hids + sizeof(unsigned) * hid0, C.hids.data(), sizeof(unsigned) * C.hids.size());
+    put(o_table + sizeof(HaloRound) * tab0, C.table.data(), sizeof(HaloRound) * C.table.size());
+    put(o_rows + sizeof(unsigned) * range[c], C.rows.data(), sizeof(unsigned) * C.rows.size());
     rec0 += C.recipe.size();
     term0 += C.terms.size();
     hid0 += C.hids.size();
+    tab0 += C.table.size();
   }
-  DFM_CUDA_TRY(put(P->d_hchunks, chunks.data(), sizeof(HaloChunk) * chunks.size()));
-  DFM_CUDA_TRY(put(P->d_ctas, desc.data(), sizeof(HaloCtaDesc) * G));
+  DFM_CUDA_TRY(cudaMalloc(&P->d_arena, at + 16));
+  P->d_blob = P->d_arena;
+  P->d_hchunks = reinterpret_cast<HaloChunk*>(P->d_arena + o_chunks);
+  P->d_ctas = reinterpret_cast<HaloCtaDesc*>(P->d_arena + o_ctas);
+  P->d_table = P->d_arena + o_table;
+  P->d_rows = reinterpret_cast<unsigned*>(P->d_arena + o_rows);
+  P->d_hids = reinterpret_cast<unsigned*>(P->d_arena + o_hids);
+  P->d_recipe = reinterpret_cast<uint4*>(P->d_arena + o_rec);
+  P->d_terms = reinterpret_cast<uint4*>(P->d_arena + o_terms);
+  DFM_CUDA_TRY(cudaMemcpyAsync(P->d_arena + arrays0, host.data(), at - arrays0, cudaMemcpyHostToDevice, s));
+  off0 = 0;
+  for (const HaloCta& C : ctas) {
+    if (!C.blob.empty())
+      DFM_CUDA_TRY(cudaMemcpyAsync(P->d_blob + off0, C.blob.data(), C.blob.size(), cudaMemcpyHostToDevice, s));
+    off0 += C.blob.size();
+  }
   P->part = part;
   P->parts = parts;
   P->merged = merge;
