@@ -210,14 +210,17 @@ k_spmv_elem(unsigned N, const unsigned* __restrict__ rowptr, const unsigned* __r
 // from global memory directly.  The copy starts at the 16-byte boundary below
 // the run and ends at the one above it (the arrays carry kArrayPad spare
 // elements).
-constexpr int kWsUnroll = 2;  // blocks per lane whose column and x loads are issued together
-constexpr int kWsChunks = 8;  // 16-byte chunks per lane and pass: a 4,096-byte slice of off-diagonal values
 
 template <int B, int LPR, typename TV>
 struct WsShape {
+  // U: blocks per lane whose column and x loads are issued together; CH: 16-byte chunks per lane and pass, the slice
+  // of off-diagonal values.  3x3 blocks at 4 lanes per row (8 rows of ~1 KB a pass) take an 8 KB slice and all of a
+  // tetrahedral row's columns at once: 75.1 us on the 200x40x40 box against 77.5 with half of both; elsewhere the
+  // larger slice costs resident warps (1x1 blocks, 160,801 rows: 12.3 against 8.3 us).
+  static constexpr int U = B == 3 && LPR == 4 ? 4 : 2, CH = B == 3 && LPR == 4 ? 16 : 8;
   static constexpr unsigned R = 32 / LPR;
   static constexpr unsigned VB = B * B * sizeof(TV);
-  static constexpr unsigned OFF = 32u * kWsChunks * 16u;
+  static constexpr unsigned OFF = 32u * CH * 16u;
   static constexpr unsigned DIAG = (R * VB + 16u + 15u) & ~15u;
   static constexpr int DCH = (int)((DIAG / 16 + 31) / 32);
   static constexpr unsigned WARP = OFF + DIAG;
@@ -263,9 +266,11 @@ k_spmv_ws(unsigned N, const unsigned* __restrict__ rowptr, const unsigned* __res
   const unsigned wpb = blockDim.x >> 5;
   const unsigned step = gridDim.x * wpb * S::R;
   double dacc = 0.0, dacc2 = 0.0;
-  for (unsigned r0 = (blockIdx.x * wpb + wi) * S::R; r0 < N; r0 += step) {
+  unsigned r0 = (blockIdx.x * wpb + wi) * S::R;
+  unsigned rp_next = r0 < N ? __ldg(rowptr + min(r0 + l, min(r0 + S::R, N))) : 0u;  // row pointers a pass ahead
+  for (; r0 < N; r0 += step) {
     const unsigned rend = min(r0 + S::R, N);
-    const unsigned rp = __ldg(rowptr + min(r0 + l, rend));
+    const unsigned rp = rp_next;
     const unsigned sb = __shfl_sync(FULL, rp, 0);
     const unsigned se = __shfl_sync(FULL, rp, S::R);
     const uintptr_t va = reinterpret_cast<uintptr_t>(off + (size_t)sb * BB);
@@ -279,36 +284,44 @@ k_spmv_ws(unsigned N, const unsigned* __restrict__ rowptr, const unsigned* __res
     const unsigned nchd = ((rend - r0) * S::VB + dd + 15u) / 16u;
     __syncwarp();  // the previous pass's reads of the slice are done
 #pragma unroll
-    for (int c = 0; c < kWsChunks; c++)
+    for (int c = 0; c < S::CH; c++)
       if (l + 32u * c < nch) ws_cp16(wv + l + 32u * c, vsrc + l + 32u * c);
 #pragma unroll
     for (int c = 0; c < S::DCH; c++)
       if (l + 32u * c < nchd) ws_cp16(wd + l + 32u * c, dsrc + l + 32u * c);
-    ws_cp_wait();
-    __syncwarp();  // every lane's copies visible to the warp
+    // the lane's blocks s0 + lane, + LPR, ... (the diagonal block last, as slot
+    // s1) in that order, U at a time: their column indices, then their
+    // x entries are requested together before the products.  The first ones
+    // are requested while the copies are in flight: after them, a pass waited
+    // for the copies, the columns and x one after another (82 us on the
+    // 200x40x40 box against the copy rate's 60).
     const unsigned i = r0 + g;
     const unsigned s0 = __shfl_sync(FULL, rp, g), s1 = __shfl_sync(FULL, rp, g + 1);
+    constexpr int U = S::U;
+    double xv[U][B];
+    auto gather = [&](unsigned sb0) {
+      unsigned col[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const unsigned s = sb0 + u * LPR;
+        col[u] = s < s1 ? __ldcs(colind + s) : i;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (sb0 + u * LPR <= s1)
+#pragma unroll
+          for (int c = 0; c < B; c++) xv[u][c] = __ldg(x + (size_t)col[u] * B + c);
+    };
+    if (i < rend) gather(s0 + lane);
+    if (r0 + step < N) rp_next = __ldg(rowptr + min(r0 + step + l, min(r0 + step + S::R, N)));
+    ws_cp_wait();
+    __syncwarp();  // every lane's copies visible to the warp
     if (i < rend) {  // group-uniform
       double acc[B];
 #pragma unroll
       for (int r = 0; r < B; r++) acc[r] = 0.0;
-      // the lane's blocks s0 + lane, + LPR, ... (the diagonal block last, as
-      // slot s1) in that order, kWsUnroll at a time: their column indices,
-      // then their x entries are requested together before the products
-      constexpr int U = kWsUnroll;
       for (unsigned sb0 = s0 + lane; sb0 <= s1; sb0 += U * LPR) {
-        unsigned col[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const unsigned s = sb0 + u * LPR;
-          col[u] = s < s1 ? __ldcs(colind + s) : i;
-        }
-        double xv[U][B];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-          if (sb0 + u * LPR <= s1)
-#pragma unroll
-            for (int c = 0; c < B; c++) xv[u][c] = __ldg(x + (size_t)col[u] * B + c);
+        if (sb0 != s0 + lane) gather(sb0);
 #pragma unroll
         for (int u = 0; u < U; u++) {
           const unsigned s = sb0 + u * LPR;

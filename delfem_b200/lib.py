@@ -168,7 +168,7 @@ def _sync_torch():
     """Order the caller's torch work (default stream) before a library call,
     which runs on the context's own stream."""
     import torch
-    if torch.cuda.is_available() and torch.cuda.is_initialized():
+    if torch.cuda.is_initialized():
         torch.cuda.current_stream().synchronize()
 
 
