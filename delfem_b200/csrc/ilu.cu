@@ -236,9 +236,15 @@ k_ilu0_factor(unsigned N, const unsigned* __restrict__ rowptr, const unsigned* _
 // reads its row of A and finds the targets of all updates before it waits, and
 // the U blocks of the rows it reads announce themselves: the factor starts out
 // as a NaN sentinel, so a value that is not one is final, as in the sweeps.
-// They are polled together, and the elimination runs from shared memory.  The
-// operations and their order are the same, so the factor is the same to the
-// bit.
+// Only blocks that have a target in the row are read at all (25 of the 49 on a
+// tetrahedral mesh), straight into registers, each lane asking again for what
+// it misses; the elimination runs from shared memory.  The operations and
+// their order are the same, so the factor is the same to the bit.
+// dfm_ilu_factor on the 200x40x40 box, copies for the sweeps included: 5.4 ms
+// with k_ilu0_factor, 2.17 ms here when every block was read in two trips,
+// 1.63 ms as it is (4,500 cycles a row for the elimination, 1,000 from the last
+// value's arrival to it); ILU(1) on 60x16x16 1.35 -> 0.69 ms.  More registers
+// for reading ahead within a row cost more in warps than they gave (1.77 ms).
 // Shared memory per warp: ucap U blocks, the row's blocks (the diagonal block
 // last) and columns, where the U blocks come from and go to.
 struct RowFactorShape {
@@ -272,7 +278,7 @@ k_ilu_factor_row(unsigned N, FactorSource src, const unsigned* __restrict__ rowp
                  RowFactorShape S) {
   static_assert(!CPLX || B == 1, "complex blocks are scalars");
   constexpr unsigned BB = CPLX ? 2 : B * B, FULL = 0xffffffffu;  // doubles per block
-  constexpr unsigned short NOT = 0xffff;
+  constexpr unsigned NOT = 0xffff, NV = 8, WIN = 64;
   extern __shared__ __align__(16) char fsmem[];
   const unsigned lane = threadIdx.x & 31u;
   char* mine = fsmem + (threadIdx.x >> 5) * S.warp_bytes;
@@ -319,62 +325,82 @@ k_ilu_factor_row(unsigned N, FactorSource src, const unsigned* __restrict__ rowp
         u0 = __ldg(diaind + k);
         len = __ldg(rowptr + k + 1) - u0;
       }
-      unsigned end = len;  // inclusive prefix sum: where the lane's U blocks end
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned t = __shfl_up_sync(FULL, end, o);
-        if (lane >= (unsigned)o) end += t;
-      }
-      const unsigned ne = (unsigned)__popc(__ballot_sync(FULL, e0 + lane < nl && end <= S.ucap));  // >= 1
-      // targets of their blocks in this row (no fill-in beyond the pattern)
-      for (unsigned e = 0; e < ne; e++) {
-        const unsigned ue = __shfl_sync(FULL, u0, (int)e), n = __shfl_sync(FULL, len, (int)e);
-        const unsigned at = __shfl_sync(FULL, end, (int)e) - n;
-        for (unsigned b = lane; b < n; b += 32) {
-          const unsigned j = __ldg(colind + ue + b);
-          unsigned lo = 0, hi = nnz;
-          while (lo < hi) {
-            const unsigned m = (lo + hi) >> 1;
-            if (rc[m] < j) lo = m + 1; else hi = m;
+      // their blocks that have a target in this row (there is no fill-in beyond the pattern), packed: lane l's
+      // lie at [at, at + n)
+      unsigned ne = 0, cnt = 0, at = 0, n = 0;
+      for (; ne < 32u && e0 + ne < nl; ne++) {
+        const unsigned ue = __shfl_sync(FULL, u0, (int)ne), ul = __shfl_sync(FULL, len, (int)ne);
+        if (cnt + ul > S.ucap) break;  // never the first: ucap holds any row's U blocks
+        if (lane == ne) at = cnt;
+        for (unsigned b0 = 0; b0 < ul; b0 += 32) {
+          const unsigned b = b0 + lane;
+          unsigned to = NOT;
+          if (b < ul) {
+            const unsigned j = __ldg(colind + ue + b);
+            unsigned lo = 0, hi = nnz;
+            while (lo < hi) {
+              const unsigned m = (lo + hi) >> 1;
+              if (rc[m] < j) lo = m + 1; else hi = m;
+            }
+            to = j == i ? nnz : lo < nnz && rc[lo] == j ? lo : NOT;
           }
-          tgt[at + b] = j == i ? (unsigned short)nnz : lo < nnz && rc[lo] == j ? (unsigned short)lo : NOT;
-          from[at + b] = ue + b;
+          const unsigned hit = __ballot_sync(FULL, to != NOT);
+          if (to != NOT) {
+            const unsigned w = cnt + (unsigned)__popc(hit & ((1u << lane) - 1u));
+            tgt[w] = (unsigned short)to;
+            from[w] = ue + b;
+          }
+          cnt += (unsigned)__popc(hit);
         }
+        if (lane == ne) n = cnt - at;
       }
       __syncwarp();
-      const unsigned total = __shfl_sync(FULL, end, (int)ne - 1) * BB;
-      // wait for the last value of each row's U blocks, then read them all (again while one is missing)
-      {
-        const double* last = lane < ne && len ? foff + (size_t)(u0 + len) * BB - 1 : nullptr;
-        SpinGuard g(wait_ns);
-        bool miss = __any_sync(FULL, last && Sent<double>::is(ld_relaxed(last)));
+      const unsigned total = cnt * BB;
+      // Values are their own flags. A lane holds NV of them; those that are missing are asked for again, first
+      // the last WIN missing ones alone (most often the row finished last), then whatever else is missing.
+      SpinGuard g(wait_ns);
+      for (unsigned q0 = 0; q0 < total; q0 += 32 * NV) {
+        double v[NV];
+#pragma unroll
+        for (unsigned k = 0; k < NV; k++) v[k] = Sent<double>::value();
+        unsigned lo = q0;
         for (;;) {
-          if (!miss) {
-            bool m = false;
-#pragma unroll 8
-            for (unsigned q = lane; q < total; q += 32) {  // all in flight together
-              const double v = ld_relaxed(foff + (size_t)from[q / BB] * BB + q % BB);
-              m |= Sent<double>::is(v);
-              uv[q] = v;
-            }
-            if (!__any_sync(FULL, m)) break;
+          int hi = -1;  // the last missing value
+#pragma unroll
+          for (unsigned k = 0; k < NV; k++) {
+            const unsigned q = q0 + 32 * k + lane;
+            if (q >= lo && q < total && Sent<double>::is(v[k]))
+              v[k] = ld_relaxed(foff + (size_t)from[q / BB] * BB + q % BB);
           }
+#pragma unroll
+          for (unsigned k = 0; k < NV; k++) {
+            const unsigned q = q0 + 32 * k + lane;
+            if (q >= lo && q < total && Sent<double>::is(v[k])) hi = (int)q;
+          }
+          hi = __reduce_max_sync(FULL, hi);
+          if (hi < 0) {
+            if (lo == q0) break;
+            lo = q0;  // the window has come: the rest
+            continue;
+          }
+          lo = (unsigned)hi >= q0 + WIN ? (unsigned)hi + 1 - WIN : q0;
           if (g.expired() || ((g.n & 1023u) == 0 && ld_status(st) != 0)) {
             raise_error(st, DFM_WAIT_TIMEOUT, 1);
             break;
           }
-          miss = __any_sync(FULL, last && Sent<double>::is(ld_relaxed(last)));
         }
+#pragma unroll
+        for (unsigned k = 0; k < NV; k++)
+          if (q0 + 32 * k + lane < total) uv[q0 + 32 * k + lane] = v[k];
       }
       __syncwarp();
       for (unsigned e = 0; e < ne; e++) {  // k ascending
-        const unsigned n = __shfl_sync(FULL, len, (int)e), at = __shfl_sync(FULL, end, (int)e) - n;
+        const unsigned en = __shfl_sync(FULL, n, (int)e), ea = __shfl_sync(FULL, at, (int)e);
         const double* l = rv + (e0 + e) * BB;
-        for (unsigned q = lane; q < n * BB; q += 32) {
+        for (unsigned q = lane; q < en * BB; q += 32) {
           const unsigned b = q / BB, el = q - b * BB;
-          const unsigned t = tgt[at + b];
-          if (t == NOT) continue;
-          rv[t * BB + el] = sub_rn(rv[t * BB + el], product(l, uv + (at + b) * BB, el));
+          const unsigned t = tgt[ea + b];
+          rv[t * BB + el] = sub_rn(rv[t * BB + el], product(l, uv + (ea + b) * BB, el));
         }
         __syncwarp();
       }
