@@ -387,8 +387,8 @@ DFM_API int dfm_ilu_apply_static(dfm_ilu M, const double* r, double* z);
  * 8 = 3 and 5 with the row groups in two halves taking alternate levels, the
  * idle half fetching its next row's operands before the level barrier (same
  * results as 3 and 5), 9 = the row ranges of 3 with the level path in shared
- * memory only: a few compute warps synchronised by a named barrier take the
- * rows of each level while producer warps stream the level data by TMA and
+ * memory only: a few compute warps synchronised by a named barrier take
+ * rounds of a level's rows while other warps stream the level data by TMA and
  * prefetch the operands owned by other CTAs into a shared-memory halo (results
  * equal to those of 3 to rounding), 10 = 9 with the levels taken in pairs as
  * in 5 (half the sequential steps; the second level reads the first level's
@@ -413,9 +413,10 @@ DFM_API int dfm_sweep_partition_patches(unsigned nnode, int ndim, const double* 
                                         unsigned* part, unsigned* nparts);
 DFM_API int dfm_ilu_get_sweep(dfm_ilu M, int* mode);
 /* No counterpart in the reference.  The launch shape of schedules 9 and 10
- * (valid while one of them is the schedule): compute warps 1, 2 or 4, lanes per row 2, 4 or 8,
- * producer warps (compute + producer <= 16).  The autotuner picks one; this
- * pins it (a row's sum runs over `lanes` lanes, so the lanes decide its
+ * (valid while one of them is the schedule): compute warps 1, 2 or 4, lanes 2, 4 or 8 per component of a
+ * row (8 runs as 4), producer warps (compute + producer <= 16; a launch has 12 warps, more producers than
+ * fit are not started).  Rebuilds the plans.  The autotuner picks one; this
+ * pins it (a component's sum runs over `lanes` lanes, so the lanes decide its
  * summation order). */
 DFM_API int dfm_ilu_set_sweep_warps(dfm_ilu M, int compute_warps, int lanes, int producer_warps);
 DFM_API int dfm_ilu_get_sweep_warps(dfm_ilu M, int* compute_warps, int* lanes, int* producer_warps);
