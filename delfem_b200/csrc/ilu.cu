@@ -384,8 +384,11 @@ k_ilu_factor_row(unsigned N, FactorSource src, const unsigned* __restrict__ rowp
             continue;
           }
           lo = (unsigned)hi >= q0 + WIN ? (unsigned)hi + 1 - WIN : q0;
-          if (g.expired() || ((g.n & 1023u) == 0 && ld_status(st) != 0)) {
-            raise_error(st, DFM_WAIT_TIMEOUT, 1);
+          // every lane counts the same looks, but has a clock and a status of its own: the warp votes and leaves
+          // together, since the loop's reductions name all lanes
+          const bool stop = g.expired() || ((g.n & 1023u) == 0 && ld_status(st) != 0);
+          if ((g.n & 63u) == 0 && __any_sync(FULL, stop)) {
+            if (lane == 0) raise_error(st, DFM_WAIT_TIMEOUT, 1);
             break;
           }
         }
