@@ -140,7 +140,8 @@ DFM_DEVINL void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 // Spins on cond() until it holds, the CTA is shutting down, or the limit runs
-// out (recorded, shutting the CTA down).  NAP: ns to sleep between looks.
+// out (recorded, shutting the CTA down).  NAP: ns to sleep between looks.  Each
+// lane leaves by itself: cond() has no vote, and the caller votes on the result.
 template <int NAP = 0, typename F>
 DFM_DEVINL bool spin_until(F cond, int* s_alive, DevStatus* st, uint64_t wait_ns, int where) {
   if (cond()) return true;
@@ -338,6 +339,21 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
           m |= halo_missing<B>(smem, reinterpret_cast<const unsigned*>(smem + P.rec + 16 * R::P)[k]);
       return m;
     };
+    // Waits until no operand of P is missing; the warp leaves together.
+    auto await_operands = [&](const I& P) {
+      SpinGuard g(wait_ns);
+      while (__any_sync(FULL, missing(P))) {
+        const bool late = g.expired();
+        if ((g.n & 15u) == 0 && __any_sync(FULL, late || !ld_volatile_i(&s_alive))) {
+          if (__any_sync(FULL, late)) {
+            if (wl == 0) raise_error(st, DFM_WAIT_TIMEOUT, 23);
+            st_volatile_i(&s_alive, 0);
+          }
+          return false;
+        }
+      }
+      return true;
+    };
     // Before round q, whose item is P: its operands; after the last round of a chunk (last) its stage is handed back
     // and the chunk after the next waited for: the last round of the next one reads a record and a table entry ahead,
     // which are in those two.  False to stop.
@@ -349,8 +365,7 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
         if (++k == K) return false;
         if (k + 2 < K) ok = await_chunk();
       }
-      if (ok && __any_sync(FULL, missing(P)))
-        ok = __all_sync(FULL, spin_until([&] { return !__any_sync(FULL, missing(P)); }, &s_alive, st, wait_ns, 23));
+      if (ok && __any_sync(FULL, missing(P))) ok = await_operands(P);
       __threadfence_block();
       return ok;
     };
@@ -561,11 +576,14 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
       if (__any_sync(FULL, got)) {
         g = SpinGuard(wait_ns);
       } else {
-        bool stop = g.expired();
-        if (stop && wl == 0) raise_error(st, DFM_WAIT_TIMEOUT, 22);
-        if (stop) st_volatile_i(&s_alive, 0);
-        if ((g.n & 15u) == 0) stop = stop || !ld_volatile_i(&s_alive);
-        if (__any_sync(FULL, stop)) break;
+        const bool late = g.expired();
+        if ((g.n & 15u) == 0 && __any_sync(FULL, late || !ld_volatile_i(&s_alive))) {
+          if (__any_sync(FULL, late)) {
+            if (wl == 0) raise_error(st, DFM_WAIT_TIMEOUT, 22);
+            st_volatile_i(&s_alive, 0);
+          }
+          break;
+        }
       }
     }
   }

@@ -3,6 +3,7 @@ and its objects go on to work with the usual limit."""
 import numpy as np
 import pytest
 
+from oracle import port as P
 from tests import cases
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +37,45 @@ def test_factor(kind):
         M.factor()
         gd, go = M.get_values()
         assert np.array_equal(gd, fd) and np.array_equal(go, fo)
+
+
+def _dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a, np.float64)).cuda()
+
+
+def _chain(N, b, cplx=False):
+    """Row i coupled with rows i - 1 and i + 1."""
+    cols = [[j for j in (i - 1, i + 1) if 0 <= j < N] for i in range(N)]
+    rp = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.uint32)
+    S = P.System(rp, np.concatenate(cols).astype(np.uint32), b, cplx=cplx)
+    S.off[:] = np.random.default_rng(b).uniform(-1.0, 1.0, S.off.size) / (4 * b)
+    S.diag[:] = np.tile([1.0, 0.5] if cplx else np.eye(b).ravel(), N)
+    return S
+
+
+@pytest.mark.parametrize("b,cplx", [(1, False), (2, False), (3, False), (1, True)])
+@pytest.mark.parametrize("warps", [(1, 2, 1), (4, 4, 8)])
+@pytest.mark.parametrize("mode", [9, 10])
+def test_halo_sweep(b, cplx, warps, mode):
+    """Eight CTAs with 2,500 rows of a chain each: a CTA waits for its predecessor's last row, 100 ns a row at the
+    least, past the limit."""
+    from delfem_b200 import lib
+    S = _chain(20000, b, cplx)
+    ctx, A, M = _make(S)
+    M.factor()
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 8, 0))
+    M.sweep = mode
+    M.sweep_warps = warps
+    _, fd, fo = S.ilu0()
+    rng = np.random.default_rng(3)
+    z = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+    for limit in (100_000, 50_000):
+        r = rng.standard_normal(S.N * S.xw)
+        ctx.set_wait_limit(limit)
+        with pytest.raises(lib.DfmError) as e:
+            M.apply(_dev(r), z)
+        assert e.value.code == lib.WAIT_TIMEOUT
+        ctx.set_wait_limit(LIMIT_NS)
+        M.apply(_dev(r), z)
+        ref = S.precond(fd, fo, r)
+        assert np.allclose(z.cpu().numpy(), ref, rtol=1e-11, atol=1e-12 * np.abs(ref).max())
