@@ -96,6 +96,10 @@ struct SpinGuard {
   DFM_DEVINL bool expired() { return ((++n & 63u) == 0) && (sm_clock() - t0 > budget); }
 };
 
+// Limit of a wait for this CTA's own copies in flight before it exits.  They land in microseconds whatever the caller's
+// limit is, and shared memory must not be given up before: the limit is far above that and not the caller's.
+constexpr uint64_t kLandNs = 1000000000ull;
+
 // ---------------------------------------------------------------- reductions
 template <int W, typename T>
 DFM_DEVINL T group_sum(T v) {

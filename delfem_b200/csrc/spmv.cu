@@ -653,7 +653,7 @@ k_spmv_tma(TmaArgs<TV> a) {
     const unsigned issued = std::min(my_tiles, consumed + (unsigned)ns);
     for (unsigned j = consumed; j < issued; j++) {
       const unsigned par = (j / (unsigned)ns) & 1u;
-      SpinGuard gd(a.wait_ns);
+      SpinGuard gd(kLandNs);
       while (!sp_try_wait(&bar[j % (unsigned)ns], par))
         if (gd.expired()) break;
     }

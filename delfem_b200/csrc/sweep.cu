@@ -384,11 +384,12 @@ k_sweep_ranges(const ChunkDesc* __restrict__ chunks, const unsigned* __restrict_
   }
   }
   if (DOT) range_dot<B, DOT, TX>(rdot, X, a0, len, true, part, rows);  // (rdot, out) over this CTA's range
-  // after an aborted wait, copies already requested must land before the CTA exits
+  // after an aborted wait, copies already requested must land before the CTA exits: the last one of every stage (an
+  // earlier one's phase is over, and its parity may be that of the phase to come, which never ends)
   if (threadIdx.x == kStageThread && !s_alive) {
-    for (unsigned q = q0; q < issued_end; q++) {
-      const unsigned k = q - q0;
-      (void)wait_stage(&bar_data[k % (unsigned)nstage], (k / (unsigned)nstage) & 1u, st, wait_ns);
+    const unsigned n = issued_end > q0 ? issued_end - q0 : 0u;
+    for (unsigned k = n > (unsigned)nstage ? n - (unsigned)nstage : 0u; k < n; k++) {
+      wait_landed(&bar_data[k % (unsigned)nstage], (k / (unsigned)nstage) & 1u, st);
     }
   }
 }
@@ -608,7 +609,7 @@ k_sweep_ranges_nb(const ChunkDesc* __restrict__ chunks, const unsigned* __restri
   if (threadIdx.x == 0)
     for (int s2 = 0; s2 < nstage; s2++) {
       const int kl = s_issued[s2];
-      if (kl >= 0) (void)wait_stage(&bar[s2], ((unsigned)kl / (unsigned)nstage) & 1u, st, wait_ns);
+      if (kl >= 0) wait_landed(&bar[s2], ((unsigned)kl / (unsigned)nstage) & 1u, st);
     }
 }
 

@@ -94,6 +94,9 @@ DFM_DEVINL bool wait_stage(uint64_t* bar, unsigned parity, DevStatus* st, uint64
   }
 }
 
+// Waits for a copy in flight before the CTA's shared memory is given up.
+DFM_DEVINL void wait_landed(uint64_t* bar, unsigned parity, DevStatus* st) { (void)wait_stage(bar, parity, st, kLandNs); }
+
 // Block partial of the CTA's share of (rdot, out) from its finished slice X.
 // DOT 1: real dot over len*B entries; DOT 2: complex matrices run as real 2x2
 // blocks (re, im per row), the unconjugated sum of rdot_i out_i with the real

@@ -268,6 +268,8 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
   __shared__ int s_alive;
   __shared__ int s_issued;  // chunks whose copy has been requested
   __shared__ int s_armed;   // halo entries that hold the sentinel or their value
+  __shared__ unsigned s_copies;              // copies requested in all
+  __shared__ unsigned s_rhs[kHaloRhsWarps];  // the first chunk whose phase that warp has not completed
   if (sc) {
     if (block_flag(&sc->done)) return;
     if (FWD && rr_part) {
@@ -463,11 +465,7 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
         par ^= 1u;
       }
     }
-    // every requested copy lands before the CTA exits; the right-hand-side
-    // warps arrive for all of them unless the CTA is shutting down
-    if (wl == 0)
-      for (unsigned k = issued > ns ? issued - ns : 0u; k < issued; k++)
-        (void)wait_stage(&landed[k % ns], (k / ns) & 1u, st, wait_ns);
+    if (wl == 0) s_copies = issued;
   } else if (warp <= ncw + kHaloRhsWarps) {
     // ---------------------------------------- right-hand sides, round table
     // a chunk's descriptor, row indices and right-hand sides are three dependent reads: the descriptor is read two
@@ -487,6 +485,7 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
       indices(cd, 0, r);
     }
     if (k0 + kHaloRhsWarps < K) cd1 = my_chunks[k0 + kHaloRhsWarps];
+    unsigned done = k0;  // the first of this warp's chunks whose phase it has not completed
     for (unsigned k = k0; k < K; k += kHaloRhsWarps) {
       HaloChunk cd2 = {};
       if (k + 2 * kHaloRhsWarps < K) cd2 = my_chunks[k + 2 * kHaloRhsWarps];
@@ -528,19 +527,18 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
             }
           }
       }
-      // (also when shutting down: the copy warp waits for the phase of every requested copy)
-      if (__all_sync(FULL, ld_volatile_i(&s_issued) > (int)k)) {
-        if (wl < nte) reinterpret_cast<uint4*>(tab)[(cd.round0 + wl) & (kHaloTable - 1)] = te;
-        __syncwarp();
-        __threadfence_block();
-        if (wl == 0) mbar_arrive(&landed[k % ns]);
-      }
       if (!ok) break;
+      if (wl < nte) reinterpret_cast<uint4*>(tab)[(cd.round0 + wl) & (kHaloTable - 1)] = te;
+      __syncwarp();
+      __threadfence_block();
+      if (wl == 0) mbar_arrive(&landed[k % ns]);
+      done = k + kHaloRhsWarps;
       cd = cd1;
       cd1 = cd2;
 #pragma unroll
       for (unsigned u = 0; u < U; u++) r[u] = r1[u];
     }
+    if (wl == 0) s_rhs[k0] = done;
   } else {
     // ---------------------------------------------------------------- halo
     // a lane takes entries first, first + step, ... and goes on to the next when one is in
@@ -587,18 +585,26 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
       }
     }
   }
-  if (DOT) {  // the CTA's partial: lanes, then compute warps in order
-    __shared__ double s_w[2][kHaloMaxCw];
-    if (warp < ncw) {
-      dre = group_sum<32>(dre);
-      dim = group_sum<32>(dim);
-      if (wl == 0) {
-        s_w[0][warp] = dre;
-        s_w[1][warp] = dim;
-      }
+  __shared__ double s_w[2][kHaloMaxCw];
+  if (DOT && warp < ncw) {  // the CTA's partial: lanes, then compute warps in order
+    dre = group_sum<32>(dre);
+    dim = group_sum<32>(dim);
+    if (wl == 0) {
+      s_w[0][warp] = dre;
+      s_w[1][warp] = dim;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // The compute warps have waited for every chunk unless the CTA is shutting down.  Then copies may still be in
+    // flight; the arrivals that their phases lack are made here, where nobody computes any more, and the copies waited
+    // for, with a limit of this wait's own.
+    if (!s_alive)
+      for (unsigned k = s_copies > ns ? s_copies - ns : 0u; k < s_copies; k++) {
+        if (k >= s_rhs[k % kHaloRhsWarps]) mbar_arrive(&landed[k % ns]);
+        wait_landed(&landed[k % ns], (k / ns) & 1u, st);
+      }
+    if (DOT) {
       dre = dim = 0.0;
       for (int w = 0; w < ncw; w++) {
         dre += s_w[0][w];

@@ -79,3 +79,31 @@ def test_halo_sweep(b, cplx, warps, mode):
         M.apply(_dev(r), z)
         ref = S.precond(fd, fo, r)
         assert np.allclose(z.cpu().numpy(), ref, rtol=1e-11, atol=1e-12 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("b,cplx", [(1, False), (3, False), (1, True)])
+@pytest.mark.parametrize("mode", [3, 9, 10])
+def test_copies_land_before_the_exit(b, cplx, mode):
+    """With a limit of 1 ns the waits for the chunks themselves may run out while copies are in flight; the CTAs wait
+    for those with a limit of their own before they exit, and do so at once (a thousand chunks a CTA)."""
+    import time
+    from delfem_b200 import lib
+    S = _chain(20000, b, cplx)
+    ctx, A, M = _make(S)
+    M.factor()
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 8, 0))
+    M.sweep = mode
+    _, fd, fo = S.ilu0()
+    r = np.random.default_rng(4).standard_normal(S.N * S.xw)
+    ref = S.precond(fd, fo, r)
+    z = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+    M.apply(_dev(r), z)
+    for _ in range(10):
+        ctx.set_wait_limit(1)
+        t0 = time.perf_counter()
+        with pytest.raises(lib.DfmError) as e:
+            M.apply(_dev(r), z)
+        assert e.value.code == lib.WAIT_TIMEOUT and time.perf_counter() - t0 < 1.0
+        ctx.set_wait_limit(LIMIT_NS)
+        M.apply(_dev(r), z)
+        assert np.allclose(z.cpu().numpy(), ref, rtol=1e-11, atol=1e-12 * np.abs(ref).max())
