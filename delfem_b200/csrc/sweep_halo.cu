@@ -116,7 +116,6 @@ struct HaloK {
   static constexpr int KT = B == 3 ? 4 : 3;
 };
 
-DFM_DEVINL unsigned ld_volatile_u(const char* p) { return *reinterpret_cast<const volatile unsigned*>(p); }
 DFM_DEVINL int ld_volatile_i(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 DFM_DEVINL void st_volatile_i(int* p, int v) { *reinterpret_cast<volatile int*>(p) = v; }
 
@@ -235,7 +234,9 @@ DFM_DEVINL void item_load(LaneItem<B, KT, TV, FWD>& P, const char* smem, const u
 
 template <int B>
 DFM_DEVINL void ld_operand(double* x, const char* p) {
-  if constexpr (B == 2) {
+  if constexpr (B == 1) {
+    x[0] = ld_volatile_s(reinterpret_cast<const double*>(p));
+  } else if constexpr (B == 2) {
     const double2 t = *reinterpret_cast<const double2*>(p);
     x[0] = t.x;
     x[1] = t.y;
@@ -245,10 +246,13 @@ DFM_DEVINL void ld_operand(double* x, const char* p) {
   }
 }
 
-// whether a halo row's value at offset o has not come yet (a row's last component is stored last)
+// Whether a halo row at offset o has not come yet: its last component, which is stored last, behind a fence.  (Places
+// of the CTA's own rows are looked at as well: they hold no sentinel.)  A value read as the same eight bytes that were
+// stored is there to stay, so rows of one component need no more; for the others the look is followed by a fence
+// before the components are read.
 template <int B>
 DFM_DEVINL bool halo_missing(const char* smem, unsigned o) {
-  return ld_volatile_u(smem + o + 8 * B - 4) == (unsigned)(DFM_SENT64 >> 32);
+  return __double2hiint(ld_volatile_s(reinterpret_cast<const double*>(smem + o) + (B - 1))) == (int)(DFM_SENT64 >> 32);
 }
 
 template <int B, int H, typename TV, bool FWD, int DOT, bool EX>
@@ -414,6 +418,7 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
         }
       }
       const bool ev = __any_sync(FULL, missing(N)) || C.last;
+      if (B > 1) __threadfence_block();
       meet(ncw);
       q++;
       return ev;
@@ -564,8 +569,12 @@ k_sweep_halo(const HaloChunk* __restrict__ chunks, const HaloCtaDesc* __restrict
         }
         if (got) {
           double* h = X + halo0 + (size_t)(ring >= E ? e : e % ring) * B;
+          if (ring < E) __threadfence_block();  // the entry was given the sentinel before this
 #pragma unroll
-          for (int c = 0; c < B; c++) st_volatile_s(h + c, v[c]);
+          for (int c = 0; c < B; c++) {
+            if (B > 1 && c == B - 1) __threadfence_block();  // the last one says that the row is there
+            st_volatile_s(h + c, v[c]);
+          }
           e += step;
           id = id1;
           id1 = e + step < E ? my_ids[e + step] : 0u;
