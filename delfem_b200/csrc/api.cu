@@ -515,6 +515,7 @@ int dfm_ilu_get_values(dfm_ilu M, double* diag, double* off, int where) {
 
 int dfm_ilu_set_values(dfm_ilu M, const double* diag, const double* off, int where) {
   if (!M) return DFM_ERR_INVALID;
+  ilu_factor_changed(M);
   int rc = copy_in(M->d_fdiag, diag, sizeof(double) * M->vw() * M->N, where, M->ctx->stream);
   if (!rc) rc = copy_in(M->d_foff, off, sizeof(double) * M->vw() * M->ncrs, where, M->ctx->stream);
   if (!rc) M->factored = true;

@@ -173,6 +173,7 @@ int spmv_autotune(dfm_mat A);
 int spmv_grid(dfm_mat A);
 // ilu.cu
 int ilu_factor_launch(dfm_ilu M, dfm_mat A);
+void ilu_factor_changed(dfm_ilu M);  // the plans' packed values are gathered again on next use
 // fill.cu
 int ilu_fill_pattern(unsigned N, const std::vector<unsigned>& rp, const std::vector<unsigned>& ci, int lev,
                      std::vector<unsigned>& frp, std::vector<unsigned>& fci, const std::vector<unsigned char>& unl,

@@ -837,6 +837,10 @@ static int factor_ctas(dfm_ilu M) {
   return (int)((rows + 7) / 8);
 }
 
+void ilu_factor_changed(dfm_ilu M) {
+  for (SweepPlan* P : {&M->plan_f, &M->plan_b, &M->plan32_f, &M->plan32_b}) P->stale = true;
+}
+
 int ilu_factor_launch(dfm_ilu M, dfm_mat A) {
   dfm_ctx c = M->ctx;
   cudaStream_t s = c->stream;
@@ -860,10 +864,7 @@ int ilu_factor_launch(dfm_ilu M, dfm_mat A) {
     }
   }
   DFM_CUDA_TRY(cudaMemsetAsync(&c->d_status->nsing, 0, sizeof(unsigned), s));
-  M->plan_f.stale = true;  // packed sweep values are re-gathered on next use
-  M->plan_b.stale = true;
-  M->plan32_f.stale = true;
-  M->plan32_b.stale = true;
+  ilu_factor_changed(M);
   M->epoch++;
   if (M->epoch == 0) {  // wrapped: clear the epochs
     DFM_CUDA_TRY(cudaMemsetAsync(M->d_flags, 0, sizeof(unsigned) * M->N, s));

@@ -145,3 +145,26 @@ def test_partition_by_chains(ctx, fill):
         rc, _, _ = lib.solve_pcg(A, M, _dev(S.rhs), x, tol=1e-10, maxit=2000)
         assert rc == lib.OK
         assert np.linalg.norm(x.cpu().numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("name", ["poisson", "solid3d", "helmholtz"])
+@pytest.mark.parametrize("mode", [1, 2, 3, 4, 5, 8, 9, 10])
+def test_factor_values_set_by_the_caller(ctx, name, mode):
+    """Applications and solves after dfm_ilu_set_values use the new factor: the schedules' packed values follow it."""
+    from delfem_b200 import lib
+    S = {"poisson": lambda: cases.poisson(30), "solid3d": lambda: cases.solid3d(12, 4, 4),
+         "helmholtz": lambda: cases.helmholtz(12, "bands")}[name]()[1]
+    A, M = _make(ctx, S)
+    M.sweep = mode
+    _, fd, fo = S.ilu0()
+    _apply(M, S, fd, fo)
+    rng = np.random.default_rng(8)
+    gd, go = fd * 0.5, fo * rng.uniform(0.2, 0.4, fo.size)
+    M.set_values(gd, go)
+    _apply(M, S, gd, go)
+    if not S.cplx:  # a solve whose preconditioner is the same factor as before: the iterations tell
+        M.set_values(fd, fo)
+        x = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+        ref = S.solve(fd, fo, tol=1e-10, maxit=2000)
+        rc, it, _ = lib.solve_pcg(A, M, _dev(S.rhs), x, tol=1e-10, maxit=2000)
+        assert rc == lib.OK and abs(int(it) - int(ref["iters"])) <= 2
