@@ -541,7 +541,7 @@ int dfm_ilu_set_sweep(dfm_ilu M, int mode) {
 
 int dfm_ilu_set_sweep_warps(dfm_ilu M, int compute_warps, int lanes, int producer_warps) {
   if (!M || (compute_warps != 1 && compute_warps != 2 && compute_warps != 4) ||
-      (lanes != 2 && lanes != 4 && lanes != 8) || producer_warps < 1 || compute_warps + producer_warps > 16)
+      (lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8) || producer_warps < 1 || compute_warps + producer_warps > 16)
     return DFM_ERR_INVALID;
   if (M->sweep != 3 || !M->plan_f.halo) return DFM_ERR_INVALID;  // modes 9 and 10 only
   const int rc = ilu_set_halo_shape(M, lanes, compute_warps);

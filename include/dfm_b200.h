@@ -413,7 +413,7 @@ DFM_API int dfm_sweep_partition_patches(unsigned nnode, int ndim, const double* 
                                         unsigned* part, unsigned* nparts);
 DFM_API int dfm_ilu_get_sweep(dfm_ilu M, int* mode);
 /* No counterpart in the reference.  The launch shape of schedules 9 and 10
- * (valid while one of them is the schedule): compute warps 1, 2 or 4, lanes 2, 4 or 8 per component of a
+ * (valid while one of them is the schedule): compute warps 1, 2 or 4, lanes 1, 2, 4 or 8 per component of a
  * row (8 runs as 4), producer warps (compute + producer <= 16; a launch has 12 warps, more producers than
  * fit are not started).  Rebuilds the plans.  The autotuner picks one; this
  * pins it (a component's sum runs over `lanes` lanes, so the lanes decide its

@@ -168,3 +168,36 @@ def test_factor_values_set_by_the_caller(ctx, name, mode):
         ref = S.solve(fd, fo, tol=1e-10, maxit=2000)
         rc, it, _ = lib.solve_pcg(A, M, _dev(S.rhs), x, tol=1e-10, maxit=2000)
         assert rc == lib.OK and abs(int(it) - int(ref["iters"])) <= 2
+
+
+@pytest.mark.parametrize("b", [1, 2, 3])
+@pytest.mark.parametrize("mode", [0, 9, 10])
+def test_the_shape_in_use_can_be_pinned(ctx, b, mode):
+    """What sweep_warps reports is accepted and gives the same bits: after the autotuner (mode 0), and for the shape
+    that a schedule starts with."""
+    S = {1: lambda: cases.poisson(60), 2: lambda: cases.solid2d(30), 3: lambda: cases.solid3d(20, 5, 5)}[b]()[1]
+    _, M = _make(ctx, S)
+    r = _dev(np.random.default_rng(6).standard_normal(S.N * S.xw))
+    z, y = torch.zeros_like(r), torch.zeros_like(r)
+    M.sweep = mode
+    M.apply(r, z)
+    if M.sweep not in (9, 10):
+        pytest.skip("the autotuner picked another schedule")
+    shape = M.sweep_warps
+    M.sweep_warps = shape
+    assert M.sweep_warps == shape
+    M.apply(r, y)
+    assert torch.equal(z, y)
+
+
+@pytest.mark.parametrize("b", [1, 3])
+@pytest.mark.parametrize("cw", [1, 2, 4])
+def test_one_lane_per_component(ctx, b, cw):
+    S = cases.poisson(40)[1] if b == 1 else cases.solid3d(14, 5, 4)[1]
+    _, M = _make(ctx, S)
+    _, fd, fo = S.ilu0()
+    for mode in (9, 10):
+        M.sweep = mode
+        M.sweep_warps = (cw, 1, 4)
+        assert M.sweep_warps == (cw, 1, 4)
+        _apply(M, S, fd, fo)
