@@ -703,13 +703,10 @@ __global__ void k_gather_halo(const HaloChunk* __restrict__ chunks, unsigned nch
   }
 }
 
-// lanes per component the kernels have for a caller's count
-static int halo_lanes(int lpr) { return std::min(lpr, 4); }
-
 int sweep_halo_refresh(dfm_ilu M, SweepPlan* P) {
   const int grid = (int)std::min<unsigned>(P->nchunks, (unsigned)M->ctx->nsm * 8);
   cudaStream_t s = M->ctx->stream;
-  const int H = halo_lanes(P->lpr);
+  const int H = P->lpr;
   const HaloRound* tab = reinterpret_cast<const HaloRound*>(P->d_table);
 #define DFM_GATHER(BV, TV, CX)                                                                                       \
   do {                                                                                                               \
@@ -793,7 +790,7 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
   const unsigned b = M->vt == DFM_COMPLEX ? 2u : M->b;  // complex scalars as real 2x2 blocks
   if (lpr == 0) lpr = b == 3 ? 2 : 1;
   if (cw == 0) cw = 2;
-  const int H = halo_lanes(lpr);
+  const int H = lpr;
   const HaloShape S = halo_shape(b, (unsigned)H, val_bytes, fwd, (unsigned)cw);
   const std::vector<unsigned>& rp = M->A->h_rowptr;
   const std::vector<unsigned>& ci = M->A->h_colind;
@@ -1312,10 +1309,12 @@ static cudaError_t launch_halo_lanes(dfm_ilu M, const SweepPlan* P, const double
 #define DFM_HALO_H(HV)                                                                                       \
   return P->extras ? launch_halo<B, HV, TV, FWD, DK, true>(M, P, in, out, rdot, part, sc, rr_part, rr_n)     \
                    : launch_halo<B, HV, TV, FWD, DK, false>(M, P, in, out, rdot, part, sc, rr_part, rr_n)
-  switch (halo_lanes(P->lpr)) {
+  switch (P->lpr) {
     case 1: DFM_HALO_H(1);
     case 2: DFM_HALO_H(2);
-    default: DFM_HALO_H(4);
+    case 4: DFM_HALO_H(4);
+    default:  // 8 lanes run when a caller asks for them: the kernel for rows of any length alone
+      return launch_halo<B, 8, TV, FWD, DK, true>(M, P, in, out, rdot, part, sc, rr_part, rr_n);
   }
 #undef DFM_HALO_H
 }

@@ -414,10 +414,10 @@ DFM_API int dfm_sweep_partition_patches(unsigned nnode, int ndim, const double* 
 DFM_API int dfm_ilu_get_sweep(dfm_ilu M, int* mode);
 /* No counterpart in the reference.  The launch shape of schedules 9 and 10
  * (valid while one of them is the schedule): compute warps 1, 2 or 4, lanes 1, 2, 4 or 8 per component of a
- * row (8 runs as 4), producer warps (compute + producer <= 16; a launch has 12 warps, more producers than
- * fit are not started).  Rebuilds the plans.  The autotuner picks one; this
- * pins it (a component's sum runs over `lanes` lanes, so the lanes decide its
- * summation order). */
+ * row, producer warps (compute + producer <= 16).  Setting it rebuilds the plans.  The autotuner picks one;
+ * this pins it (a component's sum runs over `lanes` lanes, so the lanes decide its summation order).  The
+ * getter reports the shape asked for or picked: compute warps and lanes run as reported; of the producer
+ * warps, which do not touch results, a launch starts at most 9 - compute_warps. */
 DFM_API int dfm_ilu_set_sweep_warps(dfm_ilu M, int compute_warps, int lanes, int producer_warps);
 DFM_API int dfm_ilu_get_sweep_warps(dfm_ilu M, int* compute_warps, int* lanes, int* producer_warps);
 /* Sync-free schedule knobs: cap on the number of co-resident blocks (0 = all

@@ -201,3 +201,28 @@ def test_one_lane_per_component(ctx, b, cw):
         M.sweep_warps = (cw, 1, 4)
         assert M.sweep_warps == (cw, 1, 4)
         _apply(M, S, fd, fo)
+
+
+@pytest.mark.parametrize("b", [1, 2, 3])
+@pytest.mark.parametrize("mode", [9, 10])
+@pytest.mark.parametrize("ctas", [1, 2])
+def test_lanes_set_are_the_lanes_that_run(ctx, b, mode, ctas):
+    """A row of 16 blocks whose sum tells how many lanes shared it: lane h adds blocks h, h + lanes, ..., and 1 is lost
+    beside 1e16 unless another lane has it.  Blocks 0, 4 and 8 are 1e16, 1 and -1e16: one of 8 lanes has 0 and 8,
+    another has 4; one of 4 lanes, of 2 and of 1 has all three in this order."""
+    from delfem_b200 import lib
+    S = _pattern(17, [set()] * 16 + [set(range(16))], b, 3)
+    _, M = _make(ctx, S)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+    off = np.zeros((int(S.rowptr[-1]), b, b))
+    for k, v in ((0, 1e16), (4, 1.0), (8, -1e16)):
+        off[S.rowptr[16] + k] = v * np.eye(b)
+    M.set_values(np.tile(np.eye(b).ravel(), 17), off.ravel())
+    M.sweep = mode
+    for lanes, want in ((1, 1.0), (2, 1.0), (4, 1.0), (8, 0.0)):
+        for cw in (1, 2, 4):
+            M.sweep_warps = (cw, lanes, 4)
+            z = torch.zeros(17 * b, dtype=torch.float64, device="cuda")
+            M.apply(torch.ones_like(z), z)
+            assert z.cpu().numpy().tolist() == [1.0] * (16 * b) + [want] * b, (lanes, cw)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
