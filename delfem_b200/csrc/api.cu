@@ -560,6 +560,16 @@ int dfm_ilu_get_sweep_warps(dfm_ilu M, int* compute_warps, int* lanes, int* prod
   return DFM_OK;
 }
 
+int dfm_ilu_get_sweep_info(dfm_ilu M, int backward, int fp32, dfm_sweep_info* info) {
+  if (!M || !info) return DFM_ERR_INVALID;
+  const SweepPlan& P = backward ? (fp32 ? M->plan32_b : M->plan_b) : (fp32 ? M->plan32_f : M->plan_f);
+  if (M->sweep != 3 || !P.valid || !P.halo) return DFM_ERR_INVALID;
+  const unsigned B = M->vt == DFM_COMPLEX ? 2u : M->b;
+  *info = {(unsigned)P.G, (unsigned)P.part, P.merged ? 1u : 0u, (unsigned)P.nstage, P.part_rows, P.x_slice / B,
+           P.ring, P.ringed ? 1u : 0u, P.rd_off ? 1u : 0u, P.extras ? 1u : 0u};
+  return DFM_OK;
+}
+
 int dfm_ilu_set_sweep_tuning(dfm_ilu M, int max_blocks, unsigned poll_sleep_ns) {
   if (!M || max_blocks < 0 || poll_sleep_ns > 100000) return DFM_ERR_INVALID;
   M->sweep_blocks = max_blocks;

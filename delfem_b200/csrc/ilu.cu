@@ -1076,12 +1076,12 @@ int ilu_prepare(dfm_ilu M, bool f32) {
   int rc = to_f32(M->ctx, M->d_foff, M->d_foff32, no);
   if (rc) return rc;
   if (M->sweep == 3) {
-    // FP32 plans with the FP64 plans' ranges and lanes
+    // FP32 plans with the FP64 plans' partition and lanes
     for (int f = 0; f < 2; f++) {
       SweepPlan& P64 = f ? M->plan_b : M->plan_f;
       SweepPlan& P32 = f ? M->plan32_b : M->plan32_f;
-      if (!P32.valid || P32.G != P64.G || P32.lpr != P64.lpr || P32.merged != P64.merged ||
-          P32.halo != P64.halo || P32.cw != P64.cw || P32.hw != P64.hw) {
+      if (!P32.valid || P32.G != P64.G || P32.part != P64.part || P32.parts != P64.parts || P32.lpr != P64.lpr ||
+          P32.merged != P64.merged || P32.halo != P64.halo || P32.cw != P64.cw || P32.hw != P64.hw) {
         const int G = P64.part == 2 ? P64.parts : P64.G;
         if ((rc = sweep_plan_build(M, f == 0, G, 4, 8, &P32, P64.merged, P64.part, P64.halo, P64.lpr, P64.cw)))
           return rc;

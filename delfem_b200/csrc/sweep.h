@@ -103,6 +103,8 @@ struct SweepPlan {
   unsigned x_slice = 0;             // elements of the slice (a ring) at the start of X; a zero block follows
   unsigned halo0 = 0;               // element of the halo area
   unsigned ring = 0;                // entries of the halo area
+  bool ringed = false;              // some CTA needs more, so its entries are taken over by later ones
+  unsigned part_rows = 0;           // rows of the longest part
   unsigned rd_off = 0;              // byte offset of the fused dot's vector (0: no room)
   int parts = 0;                    // parts asked for
   bool extras = false;              // some rows have more blocks than a lane's registers hold

@@ -1195,6 +1195,10 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
   P->halo0 = (unsigned)halo0;
   P->rd_off = (unsigned)sz.rd_off;
   P->ring = ring;
+  for (const HaloCta& C : ctas) {
+    P->ringed = P->ringed || C.hids.size() > ring;
+    P->part_rows = std::max(P->part_rows, (unsigned)C.rows.size());
+  }
   P->val_bytes = val_bytes;
   P->vec_bytes = 8;
   P->nstage = ns;

@@ -25,6 +25,13 @@ _lib = None
 _vp, _u, _i, _d = C.c_void_p, C.c_uint, C.c_int, C.c_double
 _up, _dp, _ip = C.POINTER(C.c_uint), C.POINTER(C.c_double), C.POINTER(C.c_int)
 
+
+class SweepInfo(C.Structure):
+    """dfm_sweep_info: what a plan of schedules 9 and 10 came out as."""
+    _fields_ = [(n, C.c_uint) for n in ("ctas", "partition", "merged", "stages", "part_rows", "slice_rows",
+                                        "halo_rows", "halo_ring", "dot_fused", "long_rows")]
+
+
 # name -> (restype, argtypes); every symbol declared in include/dfm_b200.h
 PROTOS = {
     "dfm_status_string": (C.c_char_p, [_i]),
@@ -98,6 +105,7 @@ PROTOS = {
     "dfm_ilu_get_sweep": (_i, [_vp, _ip]),
     "dfm_ilu_set_sweep_warps": (_i, [_vp, _i, _i, _i]),
     "dfm_ilu_get_sweep_warps": (_i, [_vp, _ip, _ip, _ip]),
+    "dfm_ilu_get_sweep_info": (_i, [_vp, _i, _i, C.POINTER(SweepInfo)]),
     "dfm_ilu_set_sweep_tuning": (_i, [_vp, _i, _u]),
     "dfm_ilu_set_sweep_partition": (_i, [_vp, _up, _u]),
     "dfm_sweep_partition_patches": (_i, [_u, _i, _dp, _u, _up, _up]),
@@ -587,7 +595,7 @@ class ILU:
 
     @property
     def sweep_warps(self):
-        """(compute warps, lanes per row, producer warps) of schedule 9."""
+        """(compute warps, lanes per component, producer warps) of schedules 9 and 10."""
         a, b, c = C.c_int(), C.c_int(), C.c_int()
         check(lib().dfm_ilu_get_sweep_warps(self.h, C.byref(a), C.byref(b), C.byref(c)), "dfm_ilu_get_sweep_warps")
         return a.value, b.value, c.value
@@ -595,6 +603,12 @@ class ILU:
     @sweep_warps.setter
     def sweep_warps(self, v):
         check(lib().dfm_ilu_set_sweep_warps(self.h, *(int(t) for t in v)), "dfm_ilu_set_sweep_warps")
+
+    def sweep_info(self, backward=False, fp32=False):
+        """What the plan of schedule 9 or 10 came out as (dfm_sweep_info)."""
+        info = SweepInfo()
+        check(lib().dfm_ilu_get_sweep_info(self.h, int(backward), int(fp32), C.byref(info)), "dfm_ilu_get_sweep_info")
+        return info
 
 
 class Batch:

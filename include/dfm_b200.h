@@ -420,6 +420,23 @@ DFM_API int dfm_ilu_get_sweep(dfm_ilu M, int* mode);
  * warps, which do not touch results, a launch starts at most 9 - compute_warps. */
 DFM_API int dfm_ilu_set_sweep_warps(dfm_ilu M, int compute_warps, int lanes, int producer_warps);
 DFM_API int dfm_ilu_get_sweep_warps(dfm_ilu M, int* compute_warps, int* lanes, int* producer_warps);
+/* No counterpart in the reference.  What a plan of schedules 9 and 10 came out as (the schedule's forward or
+ * backward sweep; fp32: the plan of the mixed-precision solves, made by the first of them).  DFM_ERR_INVALID
+ * where there is no such plan. */
+typedef struct dfm_sweep_info {
+  unsigned ctas;
+  unsigned partition;  /* rows of a CTA: 0 a range of the natural order, 1 a part of the caller's partition,
+                          2 a part of the partition by chains of the pattern */
+  unsigned merged;     /* steps are pairs of levels */
+  unsigned stages;     /* chunks in flight */
+  unsigned part_rows;  /* rows of the longest part */
+  unsigned slice_rows; /* rows that the slice in shared memory holds: a ring where fewer than part_rows */
+  unsigned halo_rows;  /* rows of other CTAs held */
+  unsigned halo_ring;  /* some CTA reads more of them: they are held in a ring */
+  unsigned dot_fused;  /* backward: there is room for the fused dot's vector */
+  unsigned long_rows;  /* some rows have more blocks than the lanes' registers */
+} dfm_sweep_info;
+DFM_API int dfm_ilu_get_sweep_info(dfm_ilu M, int backward, int fp32, dfm_sweep_info* info);
 /* Sync-free schedule knobs: cap on the number of co-resident blocks (0 = all
  * that fit) and the back-off between polls of a waiting lane in ns (global). */
 DFM_API int dfm_ilu_set_sweep_tuning(dfm_ilu M, int max_blocks, unsigned poll_sleep_ns);

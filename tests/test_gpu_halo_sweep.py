@@ -226,3 +226,33 @@ def test_lanes_set_are_the_lanes_that_run(ctx, b, mode, ctas):
             M.apply(torch.ones_like(z), z)
             assert z.cpu().numpy().tolist() == [1.0] * (16 * b) + [want] * b, (lanes, cw)
     lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+def test_fp32_plans_follow_the_partition(ctx):
+    """An autotuned partition by chains, a mixed solve, then ranges of the natural order with as many CTAs and the
+    same warps: the next mixed solve's plans are of those ranges."""
+    from delfem_b200 import lib
+    S = cases.solid3d(40, 12, 12)[1]
+    A, M = _make(ctx, S)
+    _, fd, fo = S.ilu0()
+    _apply(M, S, fd, fo)
+    if M.sweep not in (9, 10) or M.sweep_info().partition != 2:
+        pytest.skip("the autotuner picked no partition by chains")
+    M.sweep_warps = (2, 2, 4)
+    x = torch.zeros(S.N * 3, dtype=torch.float64, device="cuda")
+
+    def mixed():
+        rc, it, _ = lib.solve_pcg_mixed(A, M, _dev(S.rhs), x, tol=1e-8, maxit=2000)
+        assert rc == lib.OK
+        for back in (False, True):
+            d, f = M.sweep_info(back), M.sweep_info(back, fp32=True)
+            assert (f.ctas, f.partition, f.merged, f.part_rows) == (d.ctas, d.partition, d.merged, d.part_rows)
+
+    mixed()
+    mode, ctas = M.sweep, M.sweep_info().ctas
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+    M.sweep = mode
+    M.sweep_warps = (2, 2, 4)
+    assert M.sweep_info().partition == 0 and M.sweep_info().ctas == ctas
+    mixed()
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
