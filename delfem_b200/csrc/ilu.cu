@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "dfm_internal.h"
+#include "sweep_trial.h"
 
 namespace dfm {
 
@@ -1158,8 +1159,7 @@ int ilu_autotune(dfm_ilu M) {
       bool merge;
     };
     Cand top = {0, 0, 0, 0, false};
-    float top_ms = 1e30f;
-    int err = DFM_OK;
+    SweepTrials trials;
     // builds and times a candidate: its ms, or 1e30 if it cannot be built
     auto eval = [&](const Cand& c) -> float {
       SweepPlan pf, pb;
@@ -1177,9 +1177,8 @@ int ilu_autotune(dfm_ilu M) {
       const int rc = time_mode(3, &ms);
       std::swap(M->plan_f, pf);
       std::swap(M->plan_b, pb);
-      if (rc != DFM_OK && rc != DFM_ERR_UNSUPPORTED && err == DFM_OK) err = rc;
-      if (rc == DFM_OK && ms < top_ms) {
-        top_ms = ms;
+      if (rc == DFM_ERR_CUDA) cudaGetLastError();  // the launch's error ends with the candidate
+      if (trials.note(rc, ms)) {
         top = c;
         std::swap(best_f, pf);
         std::swap(best_b, pb);
@@ -1206,13 +1205,13 @@ int ilu_autotune(dfm_ilu M) {
     // better of the two while they get faster (fewer CTAs: shorter chains of hand-overs; more: shorter rounds)
     auto allowed = [&](int G) { return G <= nsm && (G == 1 || M->N >= 64u * (unsigned)G); };
     const int first = large ? nsm : M->N >= 64u * 16u ? 16 : 1;
-    const float by_chains = err ? 1e30f : eval({2, first, h0, warps_for(first), false});
-    const float by_ranges = err ? 1e30f : eval({0, first, h0, warps_for(first), false});
+    const float by_chains = trials.err ? 1e30f : eval({2, first, h0, warps_for(first), false});
+    const float by_ranges = trials.err ? 1e30f : eval({0, first, h0, warps_for(first), false});
     const int kind = by_chains <= by_ranges ? 2 : 0;
     for (const std::initializer_list<int>& side : {std::initializer_list<int>{32, 64, nsm}, {12, 8, 4, 2, 1}}) {
       float last = std::min(by_chains, by_ranges);
       for (int G : side) {
-        if (err || large || first == 1) break;
+        if (trials.err || large || first == 1) break;
         if (!allowed(G)) continue;
         const float ms = eval({kind, G, h0, warps_for(G), false});
         if (ms > last && last < 1e29f) break;
@@ -1222,31 +1221,31 @@ int ilu_autotune(dfm_ilu M) {
     if (top.G) {
       Cand c = top;
       for (int cw : {1, 2, 4})
-        if (!err && cw != c.cw && (!large || cw > c.cw / 2)) {
+        if (!trials.err && cw != c.cw && (!large || cw > c.cw / 2)) {
           Cand d = top;
           d.cw = cw;
           eval(d);
         }
-      if (!err) {
+      if (!trials.err) {
         Cand d = top;
         d.lpr = bx == 3 ? 6 - top.lpr : 3 - std::min(top.lpr, 2);  // 2 <-> 4, 1 <-> 2
         d.cw = d.lpr > top.lpr ? std::min(4, 2 * top.cw) : std::max(1, top.cw / 2);
         eval(d);
       }
-      if (!err && !large && bx < 3) {
+      if (!trials.err && !large && bx < 3) {
         Cand d = top;
         d.merge = true;
         d.lpr = 2;  // a merged row has about twice the blocks
         eval(d);
       }
     }
-    if (err) {
+    if (trials.err) {
       sweep_plan_free(&best_f);
       sweep_plan_free(&best_b);
-      return err;
+      return trials.err;
     }
-    if (top_ms < best) {
-      best = top_ms;
+    if (trials.best < best) {
+      best = trials.best;
       best_mode = 3;
       std::swap(M->plan_f, best_f);
       std::swap(M->plan_b, best_b);

@@ -84,3 +84,18 @@ def test_adapter_program_matches_oracle(demo):
     x2 = np.array(out["x_fillblk"])
     assert out["fillblk_ok"] and abs(out["fillblk_iters"] - ref2["iters"]) <= 1
     assert np.linalg.norm(x2 - ref2["x"]) <= 1e-8 * np.linalg.norm(ref2["x"])
+
+
+def test_sweep_autotuner_trials(tmp_path):
+    """A candidate whose launch fails is passed over; an expired wait ends the tuning with its status."""
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("no C++ compiler")
+    out = str(tmp_path / "sweep_trial_check")
+    r = subprocess.run([gxx, "-std=c++17", "-Wall", "-Wextra", "-Werror", "-I", os.path.join(ROOT, "include"), "-I",
+                        os.path.join(ROOT, "delfem_b200", "csrc"),
+                        os.path.join(ROOT, "tests", "cpp", "sweep_trial_check.cpp"), "-o", out],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([out], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
