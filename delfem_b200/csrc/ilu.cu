@@ -1144,9 +1144,14 @@ int ilu_autotune(dfm_ilu M) {
   // so the candidates go coordinate by coordinate: row partitions and CTA
   // counts first, at the lanes and compute warps that a level's rows suggest,
   // then other warps and lanes at the best of them, then merged level pairs.
-  // (The range schedules 3-8 were slower than this one on every system timed:
-  // 2-D Poisson 256^2, an application 412 us by mode 8 against 184 us by mode
-  // 9; they remain for callers that ask for them.)
+  // The range schedules 3-8 are slower on every mesh timed whose nodes are
+  // numbered along its lines (2-D Poisson 256^2: an application 411 us by mode
+  // 8, 170 by mode 9), where a level costs 0.2-0.9 us.  Where it costs more and
+  // rows are short they can be the faster ones (rows of 6 random neighbours
+  // within 3,000 rows, N = 100,000: 1.20 ms by mode 3, 1.63 by mode 9; a
+  // shuffled 200^2 grid 45 and 48 us), so they are timed there too; rows of
+  // more than 8 blocks were faster by mode 9 throughout (20,000 rows of ~10
+  // blocks of 3x3 within 3,000 rows: 0.49 ms against 0.68).
   {
     sweep_plan_free(&M->plan_f);
     sweep_plan_free(&M->plan_b);
@@ -1187,19 +1192,90 @@ int ilu_autotune(dfm_ilu M) {
       sweep_plan_free(&pb);
       return rc == DFM_OK ? ms : 1e30f;
     };
+    // The range schedules (3-8): one partition or CTA count after the other with every kernel and lane count (neither
+    // needs another plan), then merged pairs at the best.
+    auto eval_ranges = [&](int part, int G, bool merge, std::initializer_list<int> kinds) -> float {
+      SweepPlan pf, pb;
+      if (sweep_plan_build(M, true, G, 8, 8, &pf, merge, part) != DFM_OK ||
+          sweep_plan_build(M, false, G, 8, 8, &pb, merge, part) != DFM_OK) {
+        sweep_plan_free(&pf);
+        sweep_plan_free(&pb);
+        cudaGetLastError();
+        return 1e30f;  // the slice does not fit in shared memory
+      }
+      std::swap(M->plan_f, pf);
+      std::swap(M->plan_b, pb);
+      SweepTrials here;
+      int lpr = 0, kind = 0;
+      for (int k : kinds) {  // 0 level barrier, 1 barrier-free, 2 level barrier with the two-half row pipeline
+        if (k == 1 && !(M->plan_f.nb_ok && M->plan_b.nb_ok)) continue;
+        for (int l : {1, 2, 4, 8}) {
+          for (SweepPlan* P : {&M->plan_f, &M->plan_b}) {
+            P->lpr = l;
+            P->nb = k == 1;
+            P->pipe = k == 2;
+          }
+          float ms = 1e30f;
+          const int rc = here.err ? here.err : time_mode(3, &ms);
+          if (rc == DFM_ERR_CUDA) cudaGetLastError();
+          if (here.note(rc, ms)) {
+            lpr = l;
+            kind = k;
+          }
+        }
+      }
+      for (SweepPlan* P : {&M->plan_f, &M->plan_b}) {
+        P->lpr = std::max(1, lpr);
+        P->nb = kind == 1;
+        P->pipe = kind == 2;
+      }
+      std::swap(M->plan_f, pf);
+      std::swap(M->plan_b, pb);
+      if (here.err) {
+        trials.note(here.err, 0.f);
+      } else if (lpr && trials.note(DFM_OK, here.best)) {
+        std::swap(best_f, pf);
+        std::swap(best_b, pb);
+      }
+      sweep_plan_free(&pf);
+      sweep_plan_free(&pb);
+      return here.best;
+    };
+    const bool large = M->N > 150000;  // a plan takes tenths of a second there
+    const double mean = M->ncrs / (2.0 * M->N), held = bx == 3 ? 4.0 : 3.0;  // blocks of a row; that a lane holds
+    auto tune_ranges = [&] {
+      int part = 0, G = 0, last = 0;
+      float ms = 1e30f;
+      auto take = [&](int p, int g) {
+        const float t = trials.err ? 1e30f : eval_ranges(p, g, false, {0, 2});
+        if (t < ms) {
+          ms = t;
+          part = p;
+          G = g;
+        }
+      };
+      if (M->nparts > 0 && M->nparts <= (unsigned)nsm) take(1, (int)M->nparts);
+      for (int g : {nsm, nsm / 2, nsm / 4, 16, 8, 4, 2, 1}) {
+        if (g < 1 || g == last) continue;
+        last = g;
+        take(0, g);
+      }
+      if (G && !large && !trials.err) eval_ranges(part, G, false, {1});
+      if (G && !large && !trials.err) eval_ranges(part, G, true, {0, 1, 2});
+    };
     // rows whose blocks do not fit the lanes' registers take the slower kernel for longer rows
     unsigned long_rows = 0;
     for (unsigned i = 0; i < M->N; i++) {
       const unsigned nb = M->h_diaind[i] - M->A->h_rowptr[i], nu = M->A->h_rowptr[i + 1] - M->h_diaind[i];
       long_rows = std::max(long_rows, std::max(nb, nu));
     }
-    const int h0 = bx == 3 ? (long_rows > 8 ? 4 : 2) : (long_rows > 3 ? 2 : 1);
+    int h0 = bx == 3 ? (long_rows > 8 ? 4 : 2) : (long_rows > 3 ? 2 : 1);
+    while (h0 < 8 && mean > 2.0 * held * h0) h0 *= 2;
     const unsigned rpw = 32u / (bx * (unsigned)h0);
     auto warps_for = [&](int G) {  // a level's rows of one CTA in one round
       const double rows = 1.2 * M->N / ((double)G * nlev);
       return rows <= rpw ? 1 : rows <= 2.0 * rpw ? 2 : 4;
     };
-    const bool large = M->N > 150000;  // a plan takes tenths of a second there
     if (M->nparts > 0 && M->nparts <= (unsigned)nsm) eval({1, (int)M->nparts, h0, warps_for((int)M->nparts), false});
     // parts by chains or ranges of the natural order, compared at a middle count; then more and fewer CTAs with the
     // better of the two while they get faster (fewer CTAs: shorter chains of hand-overs; more: shorter rounds)
@@ -1218,6 +1294,15 @@ int ilu_autotune(dfm_ilu M) {
         last = ms;
       }
     }
+    // Patterns without the locality of a mesh numbered along its lines (random, banded at random, shuffled): a level
+    // costs 1-5 us where a mesh's costs 0.2-0.9, and more CTAs than a mesh's row count suggests help (5,000 rows of ~60
+    // blocks of 3x3: 0.48 ms on all SMs, 1.26 on 16).
+    auto slow_levels = [&] { return trials.best * 1e3f > 0.9f * (float)(M->nlev_f + M->nlev_b); };
+    if (!trials.err && !large && slow_levels() && !allowed(nsm)) {
+      eval({0, std::min(nsm, (int)M->N), h0, warps_for(nsm), false});
+    } else if (!trials.err && !large && slow_levels()) {
+      eval({2 - kind, nsm, h0, warps_for(nsm), false});
+    }
     if (top.G) {
       Cand c = top;
       for (int cw : {1, 2, 4})
@@ -1226,19 +1311,25 @@ int ilu_autotune(dfm_ilu M) {
           d.cw = cw;
           eval(d);
         }
+      if (!trials.err && top.cw > warps_for(top.G) && top.part != 1) {  // the partitions were compared with too few warps
+        Cand d = top;
+        d.part = 2 - top.part;
+        eval(d);
+      }
       if (!trials.err) {
         Cand d = top;
-        d.lpr = bx == 3 ? 6 - top.lpr : 3 - std::min(top.lpr, 2);  // 2 <-> 4, 1 <-> 2
+        d.lpr = top.lpr >= 4 ? top.lpr / 2 : bx == 3 ? 6 - top.lpr : 3 - top.lpr;  // 8 -> 4 -> 2, 2 -> 4 or 1, 1 -> 2
         d.cw = d.lpr > top.lpr ? std::min(4, 2 * top.cw) : std::max(1, top.cw / 2);
         eval(d);
       }
       if (!trials.err && !large && bx < 3) {
         Cand d = top;
         d.merge = true;
-        d.lpr = 2;  // a merged row has about twice the blocks
+        d.lpr = std::max(2, top.lpr);  // a merged row has about twice the blocks
         eval(d);
       }
     }
+    if (!trials.err && slow_levels() && mean <= 8.0) tune_ranges();
     if (trials.err) {
       sweep_plan_free(&best_f);
       sweep_plan_free(&best_b);

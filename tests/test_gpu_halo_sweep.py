@@ -256,3 +256,32 @@ def test_fp32_plans_follow_the_partition(ctx):
     assert M.sweep_info().partition == 0 and M.sweep_info().ctas == ctas
     mixed()
     lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+@pytest.mark.parametrize("N,k", [(5000, 30), (2000, 60)])
+def test_the_autotuner_finds_the_fast_schedules(ctx, N, k):
+    """Rows with k random neighbours on either side (no mesh): the pick is no more than a quarter slower than any
+    schedule set by hand on all SMs."""
+    from delfem_b200 import lib
+    rng = np.random.default_rng(0)
+    i, j = np.repeat(np.arange(N), k), rng.integers(0, N, N * k)
+    i, j = i[i != j], j[i != j]
+    e = np.unique(np.concatenate([i * N + j, j * N + i]))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(e // N, minlength=N))]).astype(np.uint32)
+    A = lib.Matrix(ctx, rp, (e % N).astype(np.uint32), 3)
+    A.set_values(np.tile(np.eye(3).ravel(), N), rng.uniform(-1.0, 1.0, e.size * 9) / (6 * np.diff(rp.astype(int)).max()))
+    M = lib.ILU(A)
+    M.factor()
+    r = torch.randn(3 * N, dtype=torch.float64, device="cuda")
+    z = torch.zeros_like(r)
+
+    def ms():
+        M.apply(r, z)
+        return 1e3 * min(M.time_apply(r, z, 10) for _ in range(3))
+
+    auto, pick = ms(), M.sweep
+    by_hand = {}
+    for mode in (1, 2, 3, 7, 9):
+        M.sweep = mode
+        by_hand[mode] = ms()
+    assert auto <= 1.25 * min(by_hand.values()), (auto, pick, by_hand)
