@@ -133,6 +133,7 @@ struct dfm_ilu_s {
   unsigned* d_flags = nullptr;   // per-row completion epochs of the numeric factorisation
   unsigned epoch = 0;
   unsigned max_up = ~0u;         // most blocks right of the diagonal in one row of the factor (~0: not counted yet)
+  unsigned widest = 0;           // most rows in one forward level (counted with max_up)
   double* d_tmp = nullptr;       // N*xw scratch: forward-sweep output of dfm_ilu_apply
   int sweep = 0;                 // 0 untuned, 1 sync-free grid, 2 single CTA, 3 CTA row ranges
   int sweep_blocks = 0;          // sync-free grid size cap (0 = all co-resident blocks)

@@ -831,11 +831,19 @@ static cudaError_t launch_coop(void (*fn)(KArgs...), int grid, int threads, cuda
   return launch_coop_smem(fn, grid, threads, 0, s, args...);
 }
 
-// CTAs of the factorisation, 8 rows at a time each: a few levels' rows in flight.  More would only poll rows that are
-// levels away.
+// CTAs of the factorisation, 8 rows at a time each: the rows of 12 levels in flight; more would only poll rows that are
+// levels away (5,000 rows of ~10 lower 3x3 blocks: 172 us, 180 with 17 levels).  Two things need more:
+//  * Long rows.  A row takes longer the more lower blocks it has, while the level path goes on, so from 10 blocks on
+//    the levels in flight grow with them: 20,000 scalar rows of ~100 lower blocks take 34.1 ms with 12 levels, 31.2 by
+//    k_ilu0_factor, 5.3 with 120; 5,000 rows of ~30 3x3 blocks 685 and 565 us.
+//  * Levels far wider than the average: the widest one's rows (100,000 rows of 30 blocks before a chain of 2,000: 8.6
+//    ms without, 5.8 with; 20,000 rows of 12 3x3 blocks before a chain of 4,000: 10.4 and 5.9).  A mesh's widest level
+//    is within the 12 levels.  The chain pays for the polling (100,000 rows of 2 blocks before a chain of 20,000: 27.1
+//    and 30.5 ms, 57 by k_ilu0_factor).
 static int factor_ctas(dfm_ilu M) {
-  const unsigned rows = std::min(M->N, 12 * (M->N / std::max(1u, M->nlev_f) + 1));
-  return (int)((rows + 7) / 8);
+  const double level = M->N / (double)std::max(1u, M->nlev_f) + 1.0, lower = M->ncrs / (2.0 * std::max(1u, M->N));
+  const double rows = std::min((double)M->N, std::max((double)M->widest, 12.0 * level * std::max(1.0, lower / 10.0)));
+  return (int)((rows + 7.0) / 8.0);
 }
 
 void ilu_factor_changed(dfm_ilu M) {
@@ -848,7 +856,11 @@ int ilu_factor_launch(dfm_ilu M, dfm_mat A) {
   const size_t vw = M->vw();
   if (M->max_up == ~0u) {
     M->max_up = 0;
-    for (unsigned i = 0; i < M->N; i++) M->max_up = std::max(M->max_up, M->A->h_rowptr[i + 1] - M->h_diaind[i]);
+    std::vector<unsigned> rows(M->nlev_f, 0);
+    for (unsigned i = 0; i < M->N; i++) {
+      M->max_up = std::max(M->max_up, M->A->h_rowptr[i + 1] - M->h_diaind[i]);
+      M->widest = std::max(M->widest, ++rows[M->lev_f[i]]);
+    }
   }
   const RowFactorShape S = row_factor_shape((unsigned)vw, M->A->max_row, M->max_up);
   const bool rows_fit = S.warp_bytes <= kRowFactorBytes && S.rcap < 0xffffu;

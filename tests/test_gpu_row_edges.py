@@ -93,3 +93,32 @@ def test_assembly(ctx, k, dim):
     d, o = A.get_values()
     assert np.array_equal(d, S.diag) and np.array_equal(o, S.off)
     assert np.array_equal(rhs.cpu().numpy(), S.rhs)
+
+
+@pytest.mark.parametrize("b,cplx", [(1, False), (3, False), (1, True)])
+@pytest.mark.parametrize("W,k,tail", [(4000, 3, 300), (3000, 12, 40), (300, 40, 700)])
+def test_factor_of_a_wide_level_and_a_chain(ctx, b, cplx, W, k, tail):
+    """W rows of one level, k lower blocks each, then a chain: the grid is sized by the widest level, and by the blocks
+    of a row, not by the average level."""
+    from delfem_b200 import lib
+    rng = np.random.default_rng(W)
+    first = max(4 * k, W // 8)
+    N = first + W + tail
+    rows = [set() for _ in range(N)]
+    for i in range(first, N):
+        lower = rng.choice(first, size=k, replace=False).tolist() if i < first + W else [i - 1]
+        for j in lower:
+            rows[i].add(j)
+            rows[j].add(i)
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint32)
+    S = P.System(rp, np.concatenate([np.array(sorted(r), np.uint32) for r in rows]), b, cplx=cplx)
+    S.off[:] = rng.uniform(-1.0, 1.0, S.off.size) / (4 * b * max(len(r) for r in rows))
+    S.diag[:] = np.tile([1.0, 0.5] if cplx else np.eye(b).ravel(), N)
+    A = lib.Matrix(ctx, S.rowptr, S.colind, b, lib.COMPLEX if cplx else lib.REAL)
+    A.set_values(S.diag, S.off)
+    M = lib.ILU(A)
+    rc, ns = M.factor()
+    ons, fd, fo = S.ilu0()
+    gd, go = M.get_values()
+    assert rc == lib.OK and ns == ons == 0
+    assert np.array_equal(gd, fd) and np.array_equal(go, fo)
