@@ -848,7 +848,7 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
   std::vector<HaloCta> ctas;
   // CTAs first, first + by, ...; the CTAs are independent of one another (a row's slot is set and read by its own
   // CTA), so several host threads share them
-  auto build_some = [&](int first, int by, bool ringed, unsigned chunk_bytes) -> int {
+  auto build_some = [&](int first, int by, bool ringed, unsigned chunk_bytes, unsigned round_bytes) -> int {
     std::vector<unsigned> hpos(N, NONE);                   // scratch: output row -> its halo entry
     std::vector<unsigned> hpos_in(merge ? N : 0u, NONE);   // scratch: the same for input entries
     std::vector<HaloOp> ops;
@@ -947,7 +947,7 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
           at += 16u * pieces * rd.nrow * S.B * S.H;
         }
         tab[nround - 1].shape |= kHaloLast;
-      cd.bytes = at;
+        cd.bytes = at;
         C.blob.resize(C.blob.size() + at, 0);
         char* base = C.blob.data() + cd.off;
         std::memcpy(base, C.rows.data() + pos0, 4 * (size_t)nrow);
@@ -991,14 +991,14 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
           const unsigned i = todo[p];
           if (!have_ops) row_ops(i, (unsigned)c, C.terms);
           const unsigned K = std::max(rd.K, ((unsigned)ops.size() + S.H - 1) / S.H);
-          have_ops = rd.nrow > 0 && 16u * S.pieces(K > S.KT ? K - S.KT : 0u) * (rd.nrow + 1) * S.B * S.H > kChunkMaxBytes;
+          have_ops = rd.nrow > 0 && 16u * S.pieces(K > S.KT ? K - S.KT : 0u) * (rd.nrow + 1) * S.B * S.H > round_bytes;
           if (have_ops) break;  // the row starts the next round
           p++;
           for (const HaloOp& o : ops) {
             unsigned cd;
             if (o.kind == 0) {
               cd = slot[o.v];
-            C.last[cd] = (unsigned)C.chunks.size();
+              C.last[cd] = (unsigned)C.chunks.size();
             } else {
               std::vector<unsigned>& hm = o.kind == 1 ? hpos : hpos_in;
               // fetched once; in a ring again if it was fetched more than kHaloReuse chunks ago
@@ -1007,7 +1007,7 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
                 hm[o.v] = (unsigned)C.hids.size();
                 C.hids.push_back(o.kind == 1 ? o.v : (kInput | o.v));
               }
-            cd = kHalo | hm[o.v];
+              cd = kHalo | hm[o.v];
             }
             code.push_back(cd);
             rcs.push_back(o.rc);
@@ -1034,14 +1034,14 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
     }
     return DFM_OK;
   };
-  auto build = [&](bool ringed, unsigned chunk_bytes) -> int {
+  auto build = [&](bool ringed, unsigned chunk_bytes, unsigned round_bytes) -> int {
     ctas.assign(G, HaloCta());
     // (a plan of a few thousand rows is built faster than threads are started)
     const int nt = N < 8192 ? 1 : std::min({G, 8, (int)std::max(1u, std::thread::hardware_concurrency())});
     std::vector<int> rc(nt, DFM_ERR_NOMEM);
     auto work = [&](int t) {
       try {
-        rc[t] = build_some(t, nt, ringed, chunk_bytes);
+        rc[t] = build_some(t, nt, ringed, chunk_bytes, round_bytes);
       } catch (...) {
       }
     };
@@ -1096,28 +1096,44 @@ int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* 
     return z;
   };
   // chunks of several rounds and all halo entries if enough stages fit, else a halo ring, else chunks of one round
-  Sizes sz;
-  bool built_ringed = false;
-  unsigned built_bytes = 0;
   struct Try {
     bool ringed;
-    unsigned bytes;
+    unsigned bytes, round;
   };
-  const Try tries[] = {{false, kHaloChunkBytes}, {true, kHaloChunkBytes}, {true, 1u}, {false, 1u}};
-  for (const Try& a : tries) {
-    if (sz.ns >= kHaloGoodStages) break;
-    int rc = build(a.ringed, a.bytes);
+  Sizes sz;
+  Try built = {}, now = {};
+  size_t least = SIZE_MAX;  // bytes that the areas beside the stages take at the least
+  auto attempt = [&](const Try& a) -> int {
+    now = a;
+    const int rc = build(a.ringed, a.bytes, a.round);
     if (rc) return rc;
     Sizes z;
     for (int t = kHaloMaxStages; t >= kHaloMinStages && z.ns == 0; t--) z = sizes_for(t, a.ringed);
+    least = std::min(least, z.x_bytes);
     if (z.ns > sz.ns) {
       sz = z;
-      built_ringed = a.ringed;
-      built_bytes = a.bytes;
-    } else if (sz.ns && &a == &tries[3]) {
-      rc = build(built_ringed, built_bytes);
+      built = a;
+    }
+    return DFM_OK;
+  };
+  for (const Try& a : {Try{false, kHaloChunkBytes, kChunkMaxBytes}, Try{true, kHaloChunkBytes, kChunkMaxBytes},
+                       Try{true, 1u, kChunkMaxBytes}, Try{false, 1u, kChunkMaxBytes}}) {
+    if (sz.ns >= kHaloGoodStages) break;
+    const int rc = attempt(a);
+    if (rc) return rc;
+  }
+  // Rounds of rows with hundreds of blocks may be what does not fit: smaller ones, down to a row each, as long as the
+  // other areas leave room for stages.  (With FP32 values more rows come into a round of the same bytes, so that a plan
+  // could be had in FP64 and not in FP32.)
+  for (unsigned r = kChunkMaxBytes / 2; sz.ns == 0 && r >= 256 && least + bar_bytes + kHaloMinStages * 1024 <= kHaloSmemBudget;
+       r /= 2)
+    for (const bool ringed : {true, false}) {
+      const int rc = sz.ns ? DFM_OK : attempt({ringed, 1u, r});
       if (rc) return rc;
     }
+  if (sz.ns && (now.ringed != built.ringed || now.bytes != built.bytes || now.round != built.round)) {
+    const int rc = build(built.ringed, built.bytes, built.round);
+    if (rc) return rc;
   }
   if (sz.ns == 0) return DFM_ERR_UNSUPPORTED;
   const int ns = sz.ns;

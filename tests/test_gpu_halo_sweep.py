@@ -285,3 +285,30 @@ def test_the_autotuner_finds_the_fast_schedules(ctx, N, k):
         M.sweep = mode
         by_hand[mode] = ms()
     assert auto <= 1.25 * min(by_hand.values()), (auto, pick, by_hand)
+
+
+def _read_first_rows(b):
+    """The first 64 rows are read by every later row."""
+    N = 12000 if b == 1 else 4000
+    return _pattern(N, [{i - 64, i % 64} if i >= 128 else {i - 64} if i >= 64 else set() for i in range(N)], b, 7)
+
+
+@pytest.mark.parametrize("b", [1, 2, 3])
+def test_fp32_plan_where_there_is_an_fp64_plan(ctx, b):
+    """Rows of hundreds of blocks beside a slice that holds the whole part: the mixed solve takes the schedule that
+    the FP64 one takes."""
+    from delfem_b200 import lib
+    S = _read_first_rows(b)
+    A, M = _make(ctx, S)
+    _, fd, fo = S.ilu0()
+    ref = S.solve(fd, fo, tol=1e-10, maxit=500)["x"]
+    for ctas in (1, 3):
+        lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+        M.sweep = 9
+        for solve in (lib.solve_pcg, lib.solve_pcg_mixed):
+            x = torch.zeros(S.N * b, dtype=torch.float64, device="cuda")
+            rc, _, _ = solve(A, M, _dev(S.rhs), x, tol=1e-10, maxit=500)
+            assert rc == lib.OK
+            assert np.linalg.norm(x.cpu().numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
+        assert M.sweep_info(fp32=True).ctas == M.sweep_info(backward=True, fp32=True).ctas == ctas
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
