@@ -312,3 +312,80 @@ def test_fp32_plan_where_there_is_an_fp64_plan(ctx, b):
             assert np.linalg.norm(x.cpu().numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
         assert M.sweep_info(fp32=True).ctas == M.sweep_info(backward=True, fp32=True).ctas == ctas
     lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+def _read_random_rows():
+    rng = np.random.default_rng(2)
+    return _pattern(6000, [set(rng.integers(0, i, 6).tolist()) if i else set() for i in range(6000)], 3, 9)
+
+
+# system, CTAs, what the plans must have come out as: (forward and backward, backward only)
+FORMS = {
+    "long rows 1": (lambda: cases.random_spd_like(220, 1, seed=31, density=14), 5, {"long_rows": 1}, {}),
+    "long rows 3": (lambda: cases.random_spd_like(220, 3, seed=31, density=14), 5, {"long_rows": 1}, {}),
+    "slice ring 1": (lambda: cases.poisson(90)[1], 1, {"slice ring": 1}, {}),
+    "slice ring 2": (lambda: cases.solid2d(100)[1], 2, {"slice ring": 1}, {}),
+    "slice ring 3": (lambda: cases.solid3d(100, 5, 5)[1], 8, {"slice ring": 1}, {}),
+    "fused dot over a ring": (lambda: cases.solid3d(100, 5, 5)[1], 6, {"slice ring": 1}, {"dot_fused": 1}),
+    "whole slice, separate dot": (lambda: _read_first_rows(1), 1, {"slice ring": 0}, {"dot_fused": 0}),
+    "smaller rounds": (lambda: _read_first_rows(3), 1, {}, {"dot_fused": 0, "long_rows": 1}),
+    "halo ring": (_read_random_rows, 8, {"halo_ring": 1}, {}),
+}
+
+
+@pytest.mark.parametrize("name", sorted(FORMS))
+@pytest.mark.parametrize("fp32", [False, True])
+def test_forms_of_a_plan(ctx, name, fp32):
+    """Each form of the plans, known to be the one that runs, in the application and in a PCG with FP64 or FP32
+    factor values; x to 1e-8 of the oracle's."""
+    from delfem_b200 import lib
+    make, ctas, both, backward = FORMS[name]
+    S = make()
+    A, M = _make(ctx, S)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, ctas, 0))
+    M.sweep = 9
+    _, fd, fo = S.ilu0()
+    _apply(M, S, fd, fo)
+    x = torch.zeros(S.N * S.xw, dtype=torch.float64, device="cuda")
+    solve = lib.solve_pcg_mixed if fp32 else lib.solve_pcg
+    rc, _, _ = solve(A, M, _dev(S.rhs), x, tol=1e-10, maxit=4000)
+    assert rc == lib.OK
+    for back in (False, True):
+        info = M.sweep_info(back, fp32)
+        seen = {n: getattr(info, n) for n, _ in info._fields_} | {"slice ring": int(info.slice_rows < info.part_rows)}
+        want = both | (backward if back else {})
+        assert {k: seen[k] for k in want} == want and seen["ctas"] == ctas, seen
+    if name.startswith("long rows"):  # values without symmetry, which PCG takes in its stride: A x = rhs tells
+        res = S.spmv(-1.0, x.cpu().numpy(), 1.0, S.rhs.copy())
+        assert np.linalg.norm(res) <= 1e-8 * np.linalg.norm(S.rhs)
+    else:
+        ref = S.solve(fd, fo, tol=1e-10, maxit=4000)["x"]
+        assert np.linalg.norm(x.cpu().numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
+    lib.check(lib.lib().dfm_ilu_set_sweep_tuning(M.h, 0, 0))
+
+
+
+@pytest.mark.parametrize("fill", [0, 1])
+def test_the_partition_by_chains_ran(ctx, fill):
+    """Boxes on which the autotuner picks the partition by chains: both directions' plans are of that partition, and
+    the application is the oracle's (ILU(0)) or that of the one-CTA schedule (ILU(1))."""
+    from delfem_b200 import lib
+    S = cases.solid3d(40, 12, 12)[1]
+    A = lib.Matrix(ctx, S.rowptr, S.colind, 3)
+    A.set_values(S.diag, S.off)
+    M = lib.ILU(A, fill)
+    M.factor()
+    r = np.random.default_rng(5).standard_normal(S.N * 3)
+    z, y = (torch.zeros(S.N * 3, dtype=torch.float64, device="cuda") for _ in range(2))
+    M.apply(_dev(r), z)
+    if M.sweep not in (9, 10) or M.sweep_info().partition != 2:
+        pytest.skip("the autotuner picked no partition by chains")
+    assert M.sweep_info(backward=True).partition == 2
+    if fill == 0:
+        _, fd, fo = S.ilu0()
+        ref = S.precond(fd, fo, r)
+    else:
+        M.sweep = 2
+        M.apply(_dev(r), y)
+        ref = y.cpu().numpy()
+    assert np.allclose(z.cpu().numpy(), ref, rtol=1e-11, atol=1e-12 * np.abs(ref).max())
