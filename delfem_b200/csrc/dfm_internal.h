@@ -206,9 +206,9 @@ int set_poll_sleep(unsigned ns);
 // warps cw (0: a default)
 int sweep_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, int vec_bytes, SweepPlan* P, bool merge = false,
                      int part = 0, bool halo = false, int lpr = 0, int cw = 0);
-// sweep_halo.cu
 // sweep_part.cu
 int sweep_own_partition(dfm_ilu M, unsigned G);
+// sweep_halo.cu
 int sweep_halo_plan_build(dfm_ilu M, bool fwd, int G, int val_bytes, SweepPlan* P, int part, bool merge, int H,
                           int cw);
 int sweep_halo_refresh(dfm_ilu M, SweepPlan* P);

@@ -18,8 +18,11 @@
 //  * one CTA with level barriers (mode 2): for long dependency chains with few
 //    rows per level the whole sweep runs on one SM with __syncthreads between
 //    levels, so a level costs a CTA barrier instead of a trip through L2.
-// The factorisation uses the sync-free schedule with per-row completion epochs
-// and reproduces the reference's arithmetic exactly (no FMA contraction).
+// The factorisation uses the sync-free schedule too: a row's values are their
+// own flags (k_ilu_factor_row), or, where a row does not fit in shared memory,
+// per-row completion epochs say that it is there (k_ilu0_factor,
+// k_zilu0_factor).  All reproduce the reference's arithmetic exactly (no FMA
+// contraction).
 #include <algorithm>
 
 #include "dfm_internal.h"

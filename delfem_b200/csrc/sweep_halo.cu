@@ -20,13 +20,15 @@
 //    are taken, and its round table into a ring.
 //  * Halo warps poll the other CTAs' rows in global memory (NaN sentinel = not
 //    yet written), a row per lane, in the order the rounds need them, and put
-//    them into the halo area, which holds the sentinel until then.
+//    them into the halo area, which holds the sentinel until then; a row's last
+//    component goes behind a fence and says that the row is there.
 //
 // What bounds a sweep is the chain of rounds, not bytes.  A round of one warp
 // of 1x1 rows takes 92 cycles with nothing but its loads, products, store and
 // warp barrier (measured in isolation; 115 with two warps and a named barrier,
 // 175 with four), and every other thing a compute warp does per round shows:
-// +10 the store to global memory, +18 choosing a record for lanes without a
+// +10 the store to global memory (a fence behind it, for rows of more than one
+// component, does not show in a sweep's time), +18 choosing a record for lanes without a
 // row, +32 a branch on a row's length, +44 the bookkeeping of stages, +97 a look
 // at progress counters, +110 a branch on a NaN among its operands, +150 a
 // helper warp at the barrier that does the waiting.  So the compute warps' loop
