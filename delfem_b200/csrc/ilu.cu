@@ -1122,12 +1122,23 @@ int ilu_autotune(dfm_ilu M) {
   cudaStream_t s = M->ctx->stream;
   const size_t n = (size_t)M->N * M->xw();
   double *r = nullptr, *z = nullptr;
-  DFM_CUDA_TRY(cudaMallocAsync(&r, n * sizeof(double), s));
-  DFM_CUDA_TRY(cudaMallocAsync(&z, n * sizeof(double), s));
-  DFM_CUDA_TRY(cudaMemsetAsync(r, 0, n * sizeof(double), s));
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  auto done = [&](int rc) {  // gives everything back, whatever the outcome
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    if (r) cudaFreeAsync(r, s);
+    if (z) cudaFreeAsync(z, s);
+    return rc;
+  };
+  auto prepare = [&]() -> int {
+    DFM_CUDA_TRY(cudaMallocAsync(&r, n * sizeof(double), s));
+    DFM_CUDA_TRY(cudaMallocAsync(&z, n * sizeof(double), s));
+    DFM_CUDA_TRY(cudaMemsetAsync(r, 0, n * sizeof(double), s));
+    DFM_CUDA_TRY(cudaEventCreate(&e0));
+    DFM_CUDA_TRY(cudaEventCreate(&e1));
+    return DFM_OK;
+  };
+  if (const int rc = prepare()) return done(rc);
   auto time_mode = [&](int mode, float* out_ms) -> int {
     float tmin = 1e30f;
     for (int rep = 0; rep < 4; rep++) {
@@ -1151,7 +1162,7 @@ int ilu_autotune(dfm_ilu M) {
   for (int mode = 1; mode <= 2; mode++) {
     float ms;
     int rc = time_mode(mode, &ms);
-    if (rc) return rc;
+    if (rc) return done(rc);
     if (ms < best) { best = ms; best_mode = mode; }
   }
   // The shared-memory-only schedule (modes 9 and 10; complex matrices run as
@@ -1348,7 +1359,7 @@ int ilu_autotune(dfm_ilu M) {
     if (trials.err) {
       sweep_plan_free(&best_f);
       sweep_plan_free(&best_b);
-      return trials.err;
+      return done(trials.err);
     }
     if (trials.best < best) {
       best = trials.best;
@@ -1360,10 +1371,7 @@ int ilu_autotune(dfm_ilu M) {
     sweep_plan_free(&best_b);
     M->plan_gen++;
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaFreeAsync(r, s);
-  cudaFreeAsync(z, s);
+  done(DFM_OK);
   DFM_CUDA_TRY(cudaStreamSynchronize(s));
   M->sweep = best_mode;
   M->sweep_ms = best;

@@ -107,3 +107,24 @@ def test_copies_land_before_the_exit(b, cplx, mode):
         ctx.set_wait_limit(LIMIT_NS)
         M.apply(_dev(r), z)
         assert np.allclose(z.cpu().numpy(), ref, rtol=1e-11, atol=1e-12 * np.abs(ref).max())
+
+
+def test_an_autotuner_that_times_out_gives_its_memory_back():
+    """60 applications whose tuning runs into the limit: two vectors of 1.6 MB each would be 190 MB."""
+    from delfem_b200 import lib
+    S = _chain(200000, 1)
+    ctx, A, M = _make(S)
+    M.factor()
+    r = _dev(np.random.default_rng(5).standard_normal(S.N))
+    z = torch.zeros_like(r)
+    free = []
+    for _ in range(60):
+        ctx.set_wait_limit(1)
+        with pytest.raises(lib.DfmError) as e:
+            M.apply(r, z)
+        assert e.value.code == lib.WAIT_TIMEOUT
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[4] - free[-1] < 64 << 20, free
+    ctx.set_wait_limit(LIMIT_NS)
+    M.apply(r, z)
